@@ -313,6 +313,308 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   }
 }
 
+
+// ---------------------------------------------------------------------------------------------- two query tiles per CTA
+// One CTA per SM and 256 query rows (two 128-row tiles that share every K / V tile of 128 keys). A 128 x 128 tile costs
+// 1024 tensor-pipe cycles (QK^T and PV) and 1024 cycles of the special-function pipe, and its softmax cannot start before
+// its QK^T has ended nor its PV before the softmax: with two tiles in flight the products of one run under the softmax of
+// the other. The issuer's order is  PV0_j S0_{j+1} | PV1_j S1_{j+1}.
+//   TMEM   S0 S1 (128 columns each, fp32) and O0 O1 = all 512 columns. P_t (bf16) overlays S_t and is PV's TMEM operand,
+//          so the probabilities touch no shared memory and need no proxy fence.
+//   shared Q 64 KB + a ring of 5 K / V tiles (32 KB each)
+//   warp 0 TMA, warp 1 MMA issuer, warps 4..7 / 8..11 softmax of tile 0 / 1 (one query row per thread: no shuffles);
+//   the commit behind S_{j+1} also covers PV_j, so a softmax warp that sees S_{j+1} may touch O.
+constexpr int kPairThreads = 384;
+constexpr int kPairStages = 5;
+constexpr uint32_t kPairTile = 128 * D * 2;
+constexpr int kPairSmemBytes = (2 + kPairStages) * kPairTile + 256;
+
+struct TileRange {
+  int lo, hi;   // key tiles lo .. hi (inclusive); empty when the tile lies past the end of the sequence
+};
+__device__ __forceinline__ TileRange pair_range(int q0, int T, int window) {
+  if (q0 >= T) return TileRange{1 << 30, -1};
+  return TileRange{window < 0 ? 0 : max(0, q0 - window) / 128, min(q0 + 127, T - 1) / 128};
+}
+
+// exp2(x * scale - m) of 32 scores, packed to bf16 pairs; adds the rounded values (what PV multiplies) into rs.
+__device__ __forceinline__ void exp_chunk(const uint32_t* s, uint64_t sc2, uint64_t nm2, uint32_t (&pk)[16], uint64_t (&rs)[2]) {
+#pragma unroll
+  for (int j = 0; j < 32; j += 2) {
+    const uint64_t x = fma_f32x2(pack_f32x2(__uint_as_float(s[j]), __uint_as_float(s[j + 1])), sc2, nm2);
+    float x0, x1;
+    unpack_f32x2(x, x0, x1);
+    const uint32_t pb = pack_bf16x2(exp2f(x0), exp2f(x1));
+    pk[j / 2] = pb;
+    rs[(j >> 1) & 1] = add_f32x2(rs[(j >> 1) & 1], pack_f32x2(__uint_as_float(pb << 16), __uint_as_float(pb & 0xffff0000u)));
+  }
+}
+
+__global__ void __launch_bounds__(kPairThreads, 1)
+flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                      const __grid_constant__ CUtensorMap map_v, const FwdParams p) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* sQ = smem;                          // 2 tiles
+  uint8_t* sKV = smem + 2 * kPairTile;         // K_lo V_lo K_lo+1 V_lo+1 ... through the ring
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (2 + kPairStages) * kPairTile);
+  uint64_t* q_full = bars;                     // 2
+  uint64_t* kv_full = bars + 2;                // kPairStages
+  uint64_t* kv_empty = bars + 2 + kPairStages; // kPairStages
+  uint64_t* s_full = bars + 2 + 2 * kPairStages;   // 2: S_t ready (and every earlier product of the CTA done)
+  uint64_t* p_full = s_full + 2;               // 2 x 2 (count 128): first / second 64 keys of P_t written
+  uint64_t* o_full = p_full + 4;               // 2
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n_qt = (p.T + 255) / 256;
+  const int qt = n_qt - 1 - static_cast<int>(blockIdx.x);   // heavy (late) tiles first
+  const int bh = blockIdx.y;
+  const int b = bh / p.H, h = bh - b * p.H;
+  const int q0 = qt * 256;
+  const TileRange r0 = pair_range(q0, p.T, p.window), r1 = pair_range(q0 + 128, p.T, p.window);
+  const int j_lo = r0.lo, j_hi = max(r0.hi, r1.hi);          // tile 0 always has rows
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&q_full[i], 1);
+      mbar_init(&s_full[i], 1);
+      mbar_init(&o_full[i], 1);
+      mbar_init(&p_full[2 * i], 128);
+      mbar_init(&p_full[2 * i + 1], 128);
+    }
+    for (int i = 0; i < kPairStages; ++i) {
+      mbar_init(&kv_full[i], 1);
+      mbar_init(&kv_empty[i], 1);
+    }
+    *abort_flag = 0;
+    if ((smem_u32(smem) & 1023u) != 0u) report_error(p.status, SR_ERR_BAD_ARG, 1500, 0);   // swizzle needs 1 KB alignment
+    fence_barrier_init();
+    tma_prefetch_desc(&map_q);
+    tma_prefetch_desc(&map_k);
+    tma_prefetch_desc(&map_v);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_S = tmem_base, tmem_O = tmem_base + 256;   // + 128 for tile 1
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer
+    if (elect_one()) {
+      int st = 0;
+      uint32_t ph = 1;
+      bool ok = true;
+      auto load_kv = [&](const CUtensorMap* map, int j) {
+        ok = mbar_wait(&kv_empty[st], ph, abort_flag, p.status, 1600);
+        if (!ok) return;
+        uint8_t* dst = sKV + st * kPairTile;
+        mbar_arrive_expect_tx(&kv_full[st], kPairTile);
+        tma_load_4d(dst, map, &kv_full[st], 0, h, j * 128, b);
+        tma_load_4d(dst + kQHalf, map, &kv_full[st], 64, h, j * 128, b);
+        if (++st == kPairStages) {
+          st = 0;
+          ph ^= 1u;
+        }
+      };
+      auto load_q = [&](int t) {
+        mbar_arrive_expect_tx(&q_full[t], kPairTile);
+        tma_load_4d(sQ + t * kPairTile, &map_q, &q_full[t], 0, h, q0 + t * 128, b);
+        tma_load_4d(sQ + t * kPairTile + kQHalf, &map_q, &q_full[t], 64, h, q0 + t * 128, b);
+      };
+      load_q(0);
+      load_kv(&map_k, j_lo);
+      if (r1.hi >= 0) load_q(1);
+      for (int j = j_lo; ok; ) {
+        load_kv(&map_v, j);
+        if (++j > j_hi || !ok) break;
+        load_kv(&map_k, j);
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (elect_one()) {
+      const uint32_t idesc_s = make_idesc(1, 1, 0, 0, 128, 128);   // Q (K-major) x K_j (K-major)
+      const uint32_t idesc_o = make_idesc(1, 1, 0, 1, 128, D);     // P (TMEM) x V_j (MN-major)
+      bool ok = true;
+      auto slot = [&](int n) { return sKV + (n % kPairStages) * kPairTile; };   // n-th tile of the ring
+      auto wait_slot = [&](int n, int site) {
+        ok = mbar_wait(&kv_full[n % kPairStages], (n / kPairStages) & 1u, abort_flag, p.status, site);
+        if (ok) tc_fence_after();
+        return ok;
+      };
+      auto issue_s = [&](int t, int n) {
+        const uint32_t aQ = smem_u32(sQ + t * kPairTile), aK = smem_u32(slot(n));
+        const uint32_t d = tmem_S + t * 128;
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k) {
+          const uint32_t off = (k >> 2) * kQHalf + (k & 3) * 32;
+          umma_f16_ss(d, make_smem_desc_sw128(aQ + off, 16, 1024), make_smem_desc_sw128(aK + off, 16, 1024), idesc_s, k != 0 ? 1u : 0u);
+        }
+        tc_commit(&s_full[t]);
+      };
+      int n = 0;                       // ring position of K_j; V_j is n + 1, K_{j+1} is n + 2
+      uint32_t pph0 = 0, pph1 = 0;     // phase of P_0 / P_1
+      if (wait_slot(0, 1700)) {
+        ok = mbar_wait(&q_full[0], 0, abort_flag, p.status, 1701);
+        if (ok) {
+          tc_fence_after();
+          issue_s(0, 0);
+          if (r1.hi >= 0) {
+            ok = mbar_wait(&q_full[1], 0, abort_flag, p.status, 1702);
+            if (ok && r1.lo == j_lo) {
+              tc_fence_after();
+              issue_s(1, 0);
+            }
+          }
+          if (ok) tc_commit(&kv_empty[0]);
+        }
+      }
+      for (int j = j_lo; j <= j_hi && ok; ++j, n += 2) {
+        if (!wait_slot(n + 1, 1703)) break;
+        if (j < j_hi && !wait_slot(n + 2, 1704)) break;
+        const uint32_t aV = smem_u32(slot(n + 1));
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const TileRange r = t == 0 ? r0 : r1;
+          uint32_t& pph = t == 0 ? pph0 : pph1;
+          if (j >= r.lo && j <= r.hi) {
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+              ok = mbar_wait(&p_full[2 * t + half], pph, abort_flag, p.status, 1705 + half);
+              if (!ok) break;
+              tc_fence_after();
+#pragma unroll
+              for (int k = half * 4; k < half * 4 + 4; ++k)
+                umma_f16_ts(tmem_O + t * 128, tmem_S + t * 128 + k * 8, make_smem_desc_sw128(aV + k * 2048, kQHalf, 1024), idesc_o,
+                            (j > r.lo || k != 0) ? 1u : 0u);
+            }
+            if (!ok) break;
+            pph ^= 1u;
+            if (j == r.hi) tc_commit(&o_full[t]);
+          }
+          if (j + 1 >= r.lo && j + 1 <= r.hi) issue_s(t, n + 2);   // overwrites P_t of tile j: products of one issuer run in order
+        }
+        if (!ok) break;
+        tc_commit(&kv_empty[(n + 1) % kPairStages]);
+        if (j < j_hi) tc_commit(&kv_empty[(n + 2) % kPairStages]);
+      }
+    }
+  } else if (warp >= 4) {
+    // ------------------------------------------------------------------ softmax / rescale / epilogue
+    const int t = (warp - 4) >> 2;
+    const int r = (warp & 3) * 32 + lane;       // row inside the tile == TMEM lane
+    const int qb = q0 + t * 128;                // first row of the tile
+    const int qg = qb + r;                      // global query index
+    const TileRange kr = t == 0 ? r0 : r1;
+    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t tS = tmem_S + t * 128 + lane_addr, tO = tmem_O + t * 128 + lane_addr;
+    const int k_hi = min(qg, p.T - 1);                              // last visible key
+    const int k_lo = (p.window < 0) ? 0 : max(0, qg - p.window);    // first visible key
+    const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2);
+    float m = -INFINITY, l = 0.f;
+    bool ok = true;
+    uint32_t ph = 0;
+    for (int j = kr.lo; j <= kr.hi; ++j, ph ^= 1u) {
+      ok = mbar_wait(&s_full[t], ph, abort_flag, p.status, 1800);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      uint32_t sv[128];
+#pragma unroll
+      for (int ch = 0; ch < 4; ++ch) tmem_ld_32x32(tS + ch * 32, *reinterpret_cast<uint32_t(*)[32]>(sv + ch * 32));
+      tc_wait_ld();
+      const int k0 = j * 128;
+      if (k0 + 127 > qb || (p.window >= 0 && k0 < qb + 127 - p.window)) {    // the tile is not inside the band of all its rows
+#pragma unroll
+        for (int c = 0; c < 128; ++c)
+          if (k0 + c > k_hi || k0 + c < k_lo) sv[c] = __float_as_uint(-INFINITY);
+      }
+      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int c = 0; c < 128; c += 8)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) mx4[e] = fmaxf(fmaxf(mx4[e], __uint_as_float(sv[c + e])), __uint_as_float(sv[c + 4 + e]));
+      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      // Lazy reference maximum, as in flash_fwd_kernel above: it moves only when the row maximum has grown by more than
+      // 2^kLazyLog2, so O is rescaled on almost no tile.
+      constexpr float kLazyLog2 = 8.f;
+      const float m_cand = fmaxf(m, mx * p.scale_log2);
+      const float m_new = (m == -INFINITY || m_cand - m > kLazyLog2) ? m_cand : m;
+      const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
+      const float alpha = (m == -INFINITY) ? 1.f : exp2f(m - m_use);     // nothing but zeros to rescale before the first visible key
+      m = m_new;
+      if (j > kr.lo && !__all_sync(0xffffffffu, alpha == 1.f)) {
+        l *= alpha;
+#pragma unroll 1
+        for (int ch = 0; ch < 8; ++ch) {
+          uint32_t v[16];
+          tmem_ld_32x16(tO + ch * 16, v);
+          tc_wait_ld();
+#pragma unroll
+          for (int e = 0; e < 16; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) * alpha);
+          tmem_st_32x16(tO + ch * 16, v);
+        }
+      }
+      const uint64_t nm2 = pack_f32x2(-m_use, -m_use);
+      uint64_t rs[2] = {0ull, 0ull};
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+#pragma unroll
+        for (int c2 = 0; c2 < 2; ++c2) {
+          uint32_t pk[16];
+          exp_chunk(sv + half * 64 + c2 * 32, sc2, nm2, pk, rs);
+          tmem_st_32x16(tS + half * 32 + c2 * 16, pk);
+        }
+        tc_wait_st();
+        tc_fence_before();
+        mbar_arrive(&p_full[2 * t + half]);
+      }
+      float a0, a1;
+      unpack_f32x2(add_f32x2(rs[0], rs[1]), a0, a1);
+      l += a0 + a1;
+    }
+    if (ok && kr.hi >= 0) {
+      ok = mbar_wait(&o_full[t], 0, abort_flag, p.status, 1801);
+      ok = __all_sync(0xffffffffu, ok);
+    }
+    if (ok && kr.hi >= 0) {
+      tc_fence_after();
+      const float inv = (l > 0.f) ? 1.f / l : 0.f;
+      const bool row_ok = qg < p.T;
+      __nv_bfloat16* orow = p.out + (((size_t)b * p.T + (row_ok ? qg : 0)) * p.H + h) * D;
+#pragma unroll
+      for (int ch = 0; ch < 4; ++ch) {
+        uint32_t v[32];
+        tmem_ld_32x32(tO + ch * 32, v);
+        tc_wait_ld();
+        if (row_ok) {
+#pragma unroll
+          for (int e = 0; e < 32; e += 8)
+            *reinterpret_cast<uint4*>(orow + ch * 32 + e) =
+                make_uint4(pack_bf16x2(__uint_as_float(v[e]) * inv, __uint_as_float(v[e + 1]) * inv),
+                           pack_bf16x2(__uint_as_float(v[e + 2]) * inv, __uint_as_float(v[e + 3]) * inv),
+                           pack_bf16x2(__uint_as_float(v[e + 4]) * inv, __uint_as_float(v[e + 5]) * inv),
+                           pack_bf16x2(__uint_as_float(v[e + 6]) * inv, __uint_as_float(v[e + 7]) * inv));
+        }
+      }
+      if (row_ok) p.lse[((size_t)b * p.H + h) * p.T + qg] = (l > 0.f) ? (m * 0.6931471805599453f + logf(l)) : -INFINITY;
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
 }  // namespace
 
 namespace sr_attn {
@@ -402,5 +704,14 @@ extern "C" int sr_flash_attn_fwd(const void* q, const void* k, const void* v, vo
   p.window = (window < 0 || window >= T) ? -1 : window;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = status;
-  return bkv == 64 ? launch_fwd<64>(mq, mk, mv, p, stream) : launch_fwd<128>(mq, mk, mv, p, stream);
+  if (bkv == 64) return launch_fwd<64>(mq, mk, mv, p, stream);
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(flash_fwd_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes) != cudaSuccess)
+      return -4;
+    configured = true;
+  }
+  dim3 grid((p.T + 255) / 256, p.B * p.H);
+  flash_fwd_pair_kernel<<<grid, kPairThreads, kPairSmemBytes, stream>>>(mq, mk, mv, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
