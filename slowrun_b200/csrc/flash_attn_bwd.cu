@@ -98,11 +98,6 @@ __device__ __forceinline__ void tma_reduce_add_4d(const CUtensorMap* map, const 
       ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
 }
-__device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-
 // P = exp2(S * scale_log2 - lse2) of 32 columns, in place. c_lo / c_hi: visible columns of this lane (MASK only).
 template <bool MASK>
 __device__ __forceinline__ void probabilities(uint32_t (&s)[32], const float* nlse, float scale_log2, int c_lo, int c_hi) {

@@ -31,6 +31,10 @@ struct GemmParams {
   int splitk;              // fp32 accumulate-into output: CTAs own equal shares of (tile, k-block) units and add their
                            // partial tiles with vector reductions, so the last wave is never partly idle
 
+  int k_chunks;            // splitk, pair kernel: > 0 cuts the tiles of the partial wave into this many pieces of K (WorkIter)
+  int c_tma;               // pair kernel: 1 = tiles leave through TMA stores, 2 = through TMA reduce-adds into fp32 C (Cin == C,
+                           // beta == 1), 0 = every epilogue thread stores its own row
+
   const float* row_scale;  // optional fp32 [batch, M]: output row r is scaled by row_scale[r] (before beta * Cin)
   int a_fmt, b_fmt;        // fp8 operands (kind::f8f6f4): 0 = e4m3, 1 = e5m2; ignored for bf16
 
@@ -86,12 +90,14 @@ __host__ __device__ __forceinline__ void tile_coords(const GemmParams& p, int ti
 // every worker of many problem shapes and checks that the work is covered exactly once.)
 // Work items of one CTA. Full waves of tiles are strided over the grid (concurrent CTAs work on neighbouring tiles, which
 // keeps their operand panels in L2). In splitk mode the tiles of the last, partial wave are cut along K instead: every
-// CTA gets an equal share of their (tile, k-block) units and adds its partial tile with reductions.
+// CTA gets an equal share of their (tile, k-block) units and adds its partial tile with reductions, or, with k_chunks set,
+// the items (piece of K, tile) are dealt out piece by piece.
 struct WorkIter {
   int num_kb, stride, full_tiles;
   int t;                // cursor over the strided full-wave tiles
   long long u, u_end;   // cursor / end over the tail units
   int split, v, v_end;  // column-sliced tail (tail_split mode): slices per tile, cursor and end over the slices
+  int chunk, rem;       // k_chunks mode: k-blocks per piece, tiles in the partial wave (v, v_end run over the items)
   int n_off, n_w;       // column slice of the current item within its tile (set by next())
   int bn_full;
   // worker / nworkers: this CTA (or CTA pair) and how many of them share the problem
@@ -104,6 +110,17 @@ struct WorkIter {
     bn_full = bn;
     split = 1;
     v = v_end = 0;
+    chunk = 0;
+    rem = 1;
+    if (p.splitk && p.k_chunks > 0) {
+      full_tiles = (p.num_tiles / stride) * stride;
+      rem = p.num_tiles - full_tiles;
+      chunk = (nkb + p.k_chunks - 1) / p.k_chunks;
+      v = worker;
+      v_end = rem * p.k_chunks;
+      u = u_end = 0;
+      return;
+    }
     if (!p.splitk && p.tail_split > 1) {
       split = p.tail_split;
       full_tiles = (p.num_tiles / stride) * stride;
@@ -130,6 +147,15 @@ struct WorkIter {
       kb1 = num_kb;
       partial = false;
       t += stride;
+      return true;
+    }
+    if (chunk > 0) {
+      if (v >= v_end) return false;
+      tile = full_tiles + v % rem;
+      kb0 = (v / rem) * chunk;
+      kb1 = kb0 + chunk < num_kb ? kb0 + chunk : num_kb;
+      partial = chunk < num_kb;
+      v += stride;
       return true;
     }
     if (split > 1) {
@@ -321,6 +347,21 @@ int encode_u8_map(CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t ro
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(ptr), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : report_encode_failure(r, ptr, dims, strides, box);
+}
+
+// Output map {N, M, batch} of the pair kernel's TMA epilogue: boxes of 128 bytes x 32 rows, 128B swizzle.
+int encode_out_map(CUtensorMap* map, void* ptr, bool fp32, uint64_t n, uint64_t m, uint64_t batch, uint64_t ld, uint64_t batch_stride) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (fn == nullptr) return -1;
+  const uint64_t eb = fp32 ? 4 : 2;
+  cuuint64_t dims[3] = {n, m, batch};
+  cuuint64_t strides[2] = {ld * eb, (batch > 1 ? batch_stride : m * ld) * eb};
+  cuuint32_t box[3] = {(cuuint32_t)(128 / eb), 32, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, ptr, dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : report_encode_failure(r, ptr, dims, strides, box);
 }

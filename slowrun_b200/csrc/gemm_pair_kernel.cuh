@@ -40,10 +40,11 @@ struct PairCfg {
   static constexpr int kABytes = BM * BK * 2;
   static constexpr int kBBytes = kBHalfLoad * BK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kStages = (BN == 256) ? 6 : (BN == 160 ? 7 : 8);
+  static constexpr int kStages = (BN == 256 || BN == 160) ? 6 : 8;
   static constexpr int kTmemCols = (BN == 128) ? 256 : 512;
   static constexpr int kAccStride = (BN == 128) ? 128 : 256;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
+  static constexpr int kOutBytes = 4 * 2 * 4096;                 // two 4 KB output boxes per epilogue warp
+  static constexpr int kSmemBytes = kStages * kStageBytes + kOutBytes + 1024 + 256;
   static_assert(kStageBytes % 1024 == 0, "stages must keep the 1024-byte swizzle alignment");
 };
 
@@ -119,6 +120,7 @@ __device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
 //   begin(st, p, r, row_ok)   before the first chunk
 //   chunk<BN>(st, p, f, r, c0, partial, cbase, cinbase)   f[] = alpha * accumulator for columns c0..c0+31 of row r
 //   end(st, p, r, row_ok, nj) after the last chunk of the tile in tile column nj
+//   transform(st, p, f, r, c0)   chunk() without the store, for tiles that leave through TMA (tma_out)
 struct EpiStore {
   struct Row {};
   static __device__ __forceinline__ void begin(Row&, const GemmParams&, int, bool) {}
@@ -127,18 +129,80 @@ struct EpiStore {
                                                uint8_t* cbase, const uint8_t* cinbase) {
     epilogue_store<BN, PM>(p, f, r, c0, partial, cbase, cinbase);
   }
+  static __device__ __forceinline__ void transform(Row&, const GemmParams&, float (&)[32], int, int) {}
   static __device__ __forceinline__ void end(Row&, const GemmParams&, int, bool, int) {}
 };
+
+// Output path of one epilogue warp for a tile's 32 rows: TMEM -> registers -> two alternating 4 KB boxes in shared memory
+// (32 rows x 128 bytes, 128B swizzle) -> TMA store, or TMA reduce-add for accumulate-into outputs.
+// A thread owns an output row, so its own stores would put 16 bytes into each of 32 sectors per instruction and, when
+// accumulating, wait for one DRAM round trip per 32 columns; at K <= 1024 that took longer than the tile's products. Row
+// stores -> boxes, us: [65536 x 1024] x [1024 x 3072] 338 -> 268, [8192 x 512] x [512 x 3072] 40.6 -> 27.2, weight gradient
+// [8192 x 2560]^T [8192 x 7680] 233 -> 222 (210 with the split of K below).
+template <class Epi>
+__device__ __forceinline__ void tma_out(typename Epi::Row& st, const CUtensorMap* map_c, const GemmParams& p, uint8_t* stage,
+                                        uint32_t taddr, float alpha, int c_begin, int width, int row0, int b, int lane, int& seq) {
+  const int per_box = p.c_fp32 ? 32 : 64;
+  const int nbox = width / per_box;
+#pragma unroll 1
+  for (int i = 0; i < nbox; ++i, ++seq) {
+    const int c0 = c_begin + i * per_box;
+    if (c0 >= p.N) break;
+    uint8_t* box = stage + (seq & 1) * 4096;   // seq counts the boxes of all tiles: the two take turns
+    uint8_t* row = box + lane * 128;
+    if (!p.c_fp32) {
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t v[32];
+        tmem_ld_32x32(taddr + i * 64 + half * 32, v);
+        tc_wait_ld();
+        float f[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) f[j] = alpha * __uint_as_float(v[j]);
+        if (c0 + half * 32 < p.N) Epi::transform(st, p, f, row0 + lane, c0 + half * 32);
+        if (half == 0) {
+          if (lane == 0) bulk_wait_read<1>();      // the box two steps ago has been read
+          __syncwarp();
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          *reinterpret_cast<uint4*>(row + (((half * 4 + c) ^ (lane & 7)) << 4)) =
+              make_uint4(pack_bf16x2(f[8 * c], f[8 * c + 1]), pack_bf16x2(f[8 * c + 2], f[8 * c + 3]),
+                         pack_bf16x2(f[8 * c + 4], f[8 * c + 5]), pack_bf16x2(f[8 * c + 6], f[8 * c + 7]));
+      }
+    } else {
+      uint32_t v[32];
+      tmem_ld_32x32(taddr + i * 32, v);
+      tc_wait_ld();
+      if (lane == 0) bulk_wait_read<1>();
+      __syncwarp();
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        *reinterpret_cast<float4*>(row + ((c ^ (lane & 7)) << 4)) =
+            make_float4(alpha * __uint_as_float(v[4 * c]), alpha * __uint_as_float(v[4 * c + 1]),
+                        alpha * __uint_as_float(v[4 * c + 2]), alpha * __uint_as_float(v[4 * c + 3]));
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      if (row0 < p.M) {
+        if (p.c_tma == 2) tma_reduce_add_3d(map_c, box, c0, row0, b);
+        else              tma_store_3d(map_c, box, c0, row0, b);
+      }
+      bulk_commit_group();
+    }
+  }
+}
 
 template <int BN, int EB, class Epi>
 __global__ void __launch_bounds__(kNumThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                 const GemmParams p) {
+                 const __grid_constant__ CUtensorMap map_c, const GemmParams p) {
   using C_ = PairCfg<BN>;
   constexpr int BKE = 128 / EB;   // elements of K per k-block (one 128-byte swizzle row)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C_::kStages * C_::kStageBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C_::kStages * C_::kStageBytes + C_::kOutBytes);
   uint64_t* full_bar = bars;                      // [kStages]   (used in the leader)
   uint64_t* empty_bar = bars + C_::kStages;       // [kStages]
   uint64_t* tfull_bar = bars + 2 * C_::kStages;   // [2]
@@ -166,6 +230,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     fence_barrier_init();
     tma_prefetch_desc(&map_a);
     tma_prefetch_desc(&map_b);
+    if (p.c_tma) tma_prefetch_desc(&map_c);
   }
   if (warp == 1) {
     tmem_alloc_pair(tmem_slot, C_::kTmemCols);
@@ -279,6 +344,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     int tile, kb0, kb1;
     bool partial;
     const uint32_t tempty0 = map_to_cta(smem_u32(&tempty_bar[0]), 0);
+    int out_seq = 0;
     for (; ok && wi.next(tile, kb0, kb1, partial); ++local) {
       int b, mi, nj;
       tile_coords<BN, PM>(p, tile, b, mi, nj);
@@ -296,9 +362,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       uint8_t* cbase = reinterpret_cast<uint8_t*>(p.C) + (size_t)b * p.strideC * (p.c_fp32 ? 4 : 2);
       const uint8_t* cinbase =
           p.Cin ? reinterpret_cast<const uint8_t*>(p.Cin) + (size_t)b * p.strideCin * (p.cin_fp32 ? 4 : 2) : nullptr;
-      const int nch = (wi.n_w + 31) / 32;
       typename Epi::Row st;
       Epi::begin(st, p, r, row_ok);
+      if (p.c_tma) {
+        tma_out<Epi>(st, &map_c, p, smem + C_::kStages * C_::kStageBytes + (warp - 2) * 8192, taddr, alpha, nj * BN + wi.n_off,
+                     wi.n_w, mi * PM + (int)rank * BM + q * 32, b, lane, out_seq);
+        Epi::end(st, p, r, row_ok, nj);
+        tc_fence_before();
+        mbar_arrive_cluster(tempty0 + buf * 8);
+        continue;
+      }
+      const int nch = (wi.n_w + 31) / 32;
 #pragma unroll 1
       for (int ch = 0; ch < nch; ++ch) {
         uint32_t v[32];
@@ -316,6 +390,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       tc_fence_before();
       mbar_arrive_cluster(tempty0 + buf * 8);
     }
+    if (lane == 0) bulk_wait_all();
   }
 
   // ------------------------------------------------------------ teardown
@@ -333,6 +408,24 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 template <int BN, int EB, class Epi>
 int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, int max_ctas, int allow_tail_split,
                 cudaStream_t stream) {
+  CUtensorMap mc{};
+  p.c_tma = 0;
+  if (BN != 160 && p.C != nullptr) {
+    // Tiles leave through TMA where the output is a plain store or an fp32 accumulation in place, and the tensor map can
+    // describe it. Another Cin, a bf16 accumulation (one rounding of the sum, which a reduce-add would do twice), mirrored
+    // tiles and 160-wide tiles (not a whole number of boxes) keep the row stores. TMA clips a row at 16-byte granularity, so a
+    // width that is not a multiple of 16 bytes keeps them too (it would write into the padding of the row).
+    const int eb = p.c_fp32 ? 4 : 2;
+    const bool plain = p.Cin == nullptr && !p.sym;
+    const bool accumulate = p.Cin == p.C && p.c_fp32 && p.cin_fp32 && p.beta == 1.f && !p.sym && p.ldcin == p.ldc &&
+                            (p.batch == 1 || p.strideCin == p.strideC);
+    const bool aligned = (reinterpret_cast<uintptr_t>(p.C) & 15) == 0 && (p.ldc * eb) % 16 == 0 && p.ldc >= p.N && ((long long)p.N * eb) % 16 == 0 &&
+                         (p.batch == 1 || ((p.strideC * eb) % 16 == 0 && p.strideC > 0));
+    if ((plain || accumulate) && aligned) {
+      if (int rc = encode_out_map(&mc, p.C, p.c_fp32 != 0, p.N, p.M, p.batch, p.ldc, p.strideC)) return rc;
+      p.c_tma = accumulate ? 2 : 1;
+    }
+  }
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(gemm_pair_kernel<BN, EB, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -353,10 +446,30 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, int
   if (pairs < 1) pairs = 1;
   p.tail_split = 1;
   constexpr int BKE = 128 / EB;
+  p.k_chunks = 0;
   if (p.splitk) {
-    const long long units = (long long)p.num_tiles * ((p.K + BKE - 1) / BKE);
-    if (units < pairs) pairs = (int)units;
-    if (p.num_tiles % pairs == 0) p.splitk = 0;
+    const int num_kb = (p.K + BKE - 1) / BKE;
+    const int rem = p.num_tiles % pairs;
+    if (rem == 0) {
+      p.splitk = 0;   // no partial wave: nothing to balance
+    } else {
+      // Tiles of the partial wave are cut into k_chunks pieces of K, dealt out piece by piece over all of these tiles: the
+      // pairs then walk the same stretch of K at the same time and share its operand panels in L2. (Equal contiguous shares
+      // of a tile's K per pair balance a little better but put every pair at another K: with [65536 x 3072]^T [65536 x 1024]
+      // that read 3 GB instead of 0.5 GB, 470 us against 265 us.) The count minimises rounds x
+      // (k-blocks per piece + 4), 4 k-blocks being about what the epilogue of a piece costs.
+      long long best = -1;
+      for (int s = 1; s <= num_kb && s <= 2 * pairs; ++s) {
+        const int len = (num_kb + s - 1) / s;
+        if ((num_kb + len - 1) / len != s) continue;
+        const long long cost = (long long)(((long long)rem * s + pairs - 1) / pairs) * (len + 4);
+        if (best < 0 || cost < best) {
+          best = cost;
+          p.k_chunks = s;
+        }
+      }
+      if (p.num_tiles < pairs && (long long)rem * p.k_chunks < pairs) pairs = rem * p.k_chunks;
+    }
   } else {
     // last, partial wave: when at most half of the pairs would have a tile, cut those tiles into two 128-wide
     // column slices so that the wave takes half as long
@@ -377,7 +490,7 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, int
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, gemm_pair_kernel<BN, EB, Epi>, ma, mb, p) == cudaSuccess ? 0 : -5;
+  return cudaLaunchKernelEx(&cfg, gemm_pair_kernel<BN, EB, Epi>, ma, mb, mc, p) == cudaSuccess ? 0 : -5;
 }
 
 }  // namespace

@@ -48,9 +48,7 @@ struct EpiCE {
       }
     }
   }
-  template <int BN>
-  static __device__ __forceinline__ void chunk(Row& st, const GemmParams& p, float (&f)[32], int r, int c0, bool,
-                                               uint8_t* cbase, const uint8_t*) {
+  static __device__ __forceinline__ void transform(Row& st, const GemmParams& p, float (&f)[32], int r, int c0) {
     const float cap = p.ce.cap, inv_cap = p.ce.inv_cap;
     const int V = p.ce.V;
     // target logits: rare (a chunk holds a given row's target with probability 32 / vocab), so off the main path
@@ -64,7 +62,6 @@ struct EpiCE {
         p.ce.ztgt[(size_t)r * kMaxPredict + k] = cap * tanh_approx(l * inv_cap);
       }
     }
-    __nv_bfloat16* dst = p.C ? reinterpret_cast<__nv_bfloat16*>(cbase) + (size_t)r * p.ldc + c0 : nullptr;
     float s = 0.f;
     if (c0 + 32 <= V) {
 #pragma unroll
@@ -84,6 +81,12 @@ struct EpiCE {
       }
     }
     st.sum += s;
+  }
+  template <int BN>
+  static __device__ __forceinline__ void chunk(Row& st, const GemmParams& p, float (&f)[32], int r, int c0, bool,
+                                               uint8_t* cbase, const uint8_t*) {
+    transform(st, p, f, r, c0);
+    __nv_bfloat16* dst = p.C ? reinterpret_cast<__nv_bfloat16*>(cbase) + (size_t)r * p.ldc + c0 : nullptr;
     if (dst != nullptr) {
 #pragma unroll
       for (int j = 0; j < 32; j += 8) {
