@@ -165,6 +165,161 @@ softcap_ce_kernel(__nv_bfloat16* __restrict__ logits, const long* __restrict__ t
   }
 }
 
+// ---------------------------------------------------------------------------------------------- logits as an output
+// z = cap * tanh(x / cap) of the first V columns, fp32, and its backward. Bound by memory: one pass instead of the copy,
+// division, tanh and product of the op-by-op form (4 reads and 4 writes of the fp32 logits).
+// [4096, 50257]: 595 us forward and 336 us backward against about 2900 us and 2000 us op by op.
+// tanh(u) = e / (e + 2) with e = expm1(2u): full fp32 precision also near 0, unlike the hardware tanh used above.
+__device__ __forceinline__ float tanh_exact(float u) {
+  const float a = fminf(fabsf(u), 20.f);           // tanh(20) rounds to 1
+  const float e = expm1f(2.f * a);
+  return copysignf(u != u ? u : __fdiv_rn(e, e + 2.f), u);
+}
+
+__global__ void __launch_bounds__(kThreads)
+softcap_logits_fwd_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ z, int V, long ld, float cap) {
+  const long row = blockIdx.x;
+  const __nv_bfloat16* xr = x + row * ld;
+  float* zr = z + row * V;
+#pragma unroll 4
+  for (int c = threadIdx.x; c < V; c += kThreads) {
+    const float v = __bfloat162float(xr[c]);
+    zr[c] = cap > 0.f ? cap * tanh_exact(__fdiv_rn(v, cap)) : v;
+  }
+}
+
+// dx = g * (1 - (z / cap)^2), zero in the padding columns
+__global__ void __launch_bounds__(kThreads)
+softcap_logits_bwd_kernel(const float* __restrict__ g, const float* __restrict__ z, __nv_bfloat16* __restrict__ dx, int V, int Vpad,
+                          long ld, float cap) {
+  const long row = blockIdx.x;
+  const float *gr = g + row * V, *zr = z + row * V;
+  __nv_bfloat16* dr = dx + row * ld;
+  const float inv_cap = cap > 0.f ? 1.f / cap : 0.f;
+#pragma unroll 4
+  for (int c = threadIdx.x; c < Vpad; c += kThreads) {
+    float d = 0.f;
+    if (c < V) {
+      const float t = zr[c] * inv_cap;
+      d = gr[c] * (1.f - t * t);
+    }
+    dr[c] = __float2bfloat16(d);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------- distillation
+// Cross-entropy (label smoothing `ls`) and KL(teacher / T || student / T) of fp32 logits, one CTA per row, and their
+// gradient. The rows are read twice in the forward (the second time from L2) and once in the backward; nothing of the size
+// of the logits is written but the gradient. [4096, 50257]: 560 us forward and 395 us backward against about 10 ms op by op.
+constexpr int kDistThreads = 512;
+
+struct MaxSum {   // sum of exp(v - m) over what has been seen; m = maximum
+  float m, s;
+};
+__device__ __forceinline__ float exp_nat(float x) { return exp2f(x * 1.4426950408889634f); }
+__device__ __forceinline__ void add_value(MaxSum& a, float v) {
+  if (v > a.m) {
+    a.s = a.s * exp_nat(a.m - v) + 1.f;
+    a.m = v;
+  } else {
+    a.s += exp_nat(v - a.m);
+  }
+}
+__device__ __forceinline__ MaxSum merge(MaxSum a, MaxSum b) {
+  const float m = fmaxf(a.m, b.m);
+  return MaxSum{m, (a.m == -INFINITY ? 0.f : a.s * exp_nat(a.m - m)) + (b.m == -INFINITY ? 0.f : b.s * exp_nat(b.m - m))};
+}
+__device__ __forceinline__ float block_sum(float v, float* red) {
+  __syncthreads();
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  float t = 0.f;
+  for (int i = 0; i < kDistThreads / 32; ++i) t += red[i];
+  return t;
+}
+__device__ __forceinline__ float block_lse(MaxSum v, MaxSum* red) {
+  __syncthreads();
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    v = merge(v, MaxSum{__shfl_xor_sync(0xffffffffu, v.m, o), __shfl_xor_sync(0xffffffffu, v.s, o)});
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  MaxSum t = red[0];
+  for (int i = 1; i < kDistThreads / 32; ++i) t = merge(t, red[i]);
+  return t.m + static_cast<float>(log(static_cast<double>(t.s)));   // once per row; the fast single-precision log is off by 2^-21
+}
+
+// stats: [3, M] log-sum-exp of s, s / T and t / T; ce, kl: [M] (0 for ignored rows)
+__global__ void __launch_bounds__(kDistThreads)
+distill_fwd_kernel(const float* __restrict__ s, const float* __restrict__ t, const long* __restrict__ y, float* __restrict__ ce,
+                   float* __restrict__ kl, float* __restrict__ stats, long M, int V, float inv_T, float ls) {
+  __shared__ MaxSum red[kDistThreads / 32];
+  __shared__ float red1[kDistThreads / 32];
+  const long row = blockIdx.x;
+  const long target = y[row];
+  if (target == -1) {
+    if (threadIdx.x == 0) ce[row] = kl[row] = stats[row] = stats[M + row] = stats[2 * M + row] = 0.f;
+    return;
+  }
+  const float *sr = s + row * V, *tr = t + row * V;
+  const bool same = inv_T == 1.f;
+  MaxSum a{-INFINITY, 0.f}, b{-INFINITY, 0.f}, c{-INFINITY, 0.f};
+  float sum = 0.f;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < V; i += kDistThreads) {
+    const float x = sr[i], u = tr[i];
+    add_value(a, x);
+    if (!same) add_value(b, x * inv_T);
+    add_value(c, u * inv_T);
+    sum += x;
+  }
+  const float l1 = block_lse(a, red), lt = block_lse(c, red), lT = same ? l1 : block_lse(b, red);
+  float k = 0.f;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < V; i += kDistThreads) {
+    const float lp = tr[i] * inv_T - lt;
+    k += exp_nat(lp) * (lp - (sr[i] * inv_T - lT));
+  }
+  k = block_sum(k, red1);
+  sum = ls > 0.f ? block_sum(sum, red1) : 0.f;
+  if (threadIdx.x == 0) {
+    const bool ok = target >= 0 && target < V;
+    const float nll = ok ? l1 - sr[target] : __int_as_float(0x7fc00000);     // a target outside the vocabulary: NaN
+    ce[row] = (1.f - ls) * nll + (ls > 0.f ? ls * (l1 - sum / (float)V) : 0.f);
+    kl[row] = k;
+    stats[row] = l1;
+    stats[M + row] = lT;
+    stats[2 * M + row] = lt;
+  }
+}
+
+// ds = g_ce / N * (softmax(s) - target distribution) + g_kl / (N T) * (softmax(s / T) - softmax(t / T))
+__global__ void __launch_bounds__(kDistThreads)
+distill_bwd_kernel(const float* __restrict__ s, const float* __restrict__ t, const long* __restrict__ y, const float* __restrict__ stats,
+                   const float* __restrict__ n_valid, const float* __restrict__ g_ce, const float* __restrict__ g_kl,
+                   float* __restrict__ ds, long M, int V, float inv_T, float ls) {
+  const long row = blockIdx.x;
+  const long target = y[row];
+  const float *sr = s + row * V, *tr = t + row * V;
+  float* dr = ds + row * V;
+  if (target == -1) {
+    for (int i = threadIdx.x; i < V; i += kDistThreads) dr[i] = 0.f;
+    return;
+  }
+  const float l1 = stats[row], lT = stats[M + row], lt = stats[2 * M + row];
+  const float wc = *g_ce / *n_valid, wk = *g_kl / *n_valid * inv_T, base = ls / (float)V;
+  const bool same = inv_T == 1.f;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < V; i += kDistThreads) {
+    const float x = sr[i];
+    const float p1 = exp_nat(x - l1), pT = same ? p1 : exp_nat(x * inv_T - lT), pt = exp_nat(tr[i] * inv_T - lt);
+    const float q = base + (i == target ? 1.f - ls : 0.f);
+    dr[i] = wc * (p1 - q) + wk * (pT - pt);
+  }
+}
+
 }  // namespace
 
 // logits: [M, ld] bf16 (ld >= Vpad, Vpad % 8 == 0), overwritten with the gradient when write_grad != 0.
@@ -177,5 +332,36 @@ extern "C" int sr_softcap_ce(void* logits, const long* targets, float* loss, con
   if (Vpad % 8 || ld % 8 || n_predict < 1 || n_predict > kMaxPredict || V > Vpad) return -2;
   softcap_ce_kernel<<<(unsigned)M, kThreads, 0, s>>>(reinterpret_cast<__nv_bfloat16*>(logits), targets, loss, weights,
                                                      n_predict, scale_ptr, M, Vpad, V, ld, cap, write_grad);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
+// x: bf16 [M, ld]; z: fp32 [M, V] contiguous. cap <= 0: z = x.
+extern "C" int sr_softcap_logits_fwd(const void* x, float* z, long M, int V, long ld, float cap, cudaStream_t s) {
+  if (M <= 0 || V <= 0) return 0;
+  if (ld < V || M > 0x7fffffffL) return -2;
+  softcap_logits_fwd_kernel<<<(unsigned)M, kThreads, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), z, V, ld, cap);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+// g, z: fp32 [M, V] contiguous; dx: bf16 [M, ld], columns 0 .. Vpad - 1 written.
+extern "C" int sr_softcap_logits_bwd(const float* g, const float* z, void* dx, long M, int V, int Vpad, long ld, float cap, cudaStream_t s) {
+  if (M <= 0 || Vpad <= 0) return 0;
+  if (ld < Vpad || V > Vpad || M > 0x7fffffffL) return -2;
+  softcap_logits_bwd_kernel<<<(unsigned)M, kThreads, 0, s>>>(g, z, reinterpret_cast<__nv_bfloat16*>(dx), V, Vpad, ld, cap);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+// s, t: fp32 [M, V] contiguous; y: int64 [M], -1 = ignored; ce, kl: fp32 [M]; stats: fp32 [3, M].
+extern "C" int sr_distill_fwd(const float* s, const float* t, const long* y, float* ce, float* kl, float* stats, long M, int V, float T,
+                              float label_smoothing, cudaStream_t st) {
+  if (M <= 0) return 0;
+  if (V <= 0 || M > 0x7fffffffL) return -2;
+  distill_fwd_kernel<<<(unsigned)M, kDistThreads, 0, st>>>(s, t, y, ce, kl, stats, M, V, 1.f / T, label_smoothing);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+// n_valid, g_ce, g_kl: device fp32 scalars (number of rows that count; gradients of the two means); ds: fp32 [M, V].
+extern "C" int sr_distill_bwd(const float* s, const float* t, const long* y, const float* stats, const float* n_valid, const float* g_ce,
+                              const float* g_kl, float* ds, long M, int V, float T, float label_smoothing, cudaStream_t st) {
+  if (M <= 0) return 0;
+  if (V <= 0 || M > 0x7fffffffL) return -2;
+  distill_bwd_kernel<<<(unsigned)M, kDistThreads, 0, st>>>(s, t, y, stats, n_valid, g_ce, g_kl, ds, M, V, 1.f / T, label_smoothing);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

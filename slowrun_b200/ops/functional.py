@@ -11,6 +11,7 @@ import math
 import torch
 import torch.nn.functional as F
 from torch.autograd import Function
+from torch.autograd.function import once_differentiable
 
 from . import _lib
 from .gemm import gemm
@@ -663,10 +664,43 @@ def lm_head_rows(x, w, targets, cap, vocab, w_t=False):
     return softcap_ce_ref(logits.reshape(-1, logits.size(-1)), targets.reshape(-1), cap, vocab, None, "none")
 
 
+class _SoftcapLogitsFn(Function):
+    """fp32 cap * tanh(x / cap) of the first `vocab` columns of bf16 logits [..., padded vocabulary]."""
+
+    @staticmethod
+    def forward(ctx, x, cap, vocab):
+        x2 = _c(x.reshape(-1, x.size(-1)))
+        z = torch.empty((x2.size(0), vocab), dtype=torch.float32, device=x.device)
+        _call("sr_softcap_logits_fwd", [c_void_p, c_void_p, c_long, c_int, c_long, c_float, c_void_p], x2.data_ptr(), z.data_ptr(),
+              x2.size(0), vocab, x2.stride(0), cap, _lib.stream_ptr())
+        z = z.view(*x.shape[:-1], vocab)
+        ctx.cap, ctx.shape = cap, x.shape
+        ctx.save_for_backward(z)
+        return z
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, g):
+        (z,) = ctx.saved_tensors
+        g = _c(g)
+        dx = torch.empty(ctx.shape, dtype=torch.bfloat16, device=g.device)
+        Vpad = ctx.shape[-1]
+        _call("sr_softcap_logits_bwd", [c_void_p] * 3 + [c_long, c_int, c_int, c_long, c_float, c_void_p], g.data_ptr(), z.data_ptr(),
+              dx.data_ptr(), dx.numel() // max(Vpad, 1), z.size(-1), Vpad, Vpad, ctx.cap, _lib.stream_ptr())
+        return dx, None, None
+
+
+def _softcap_logits(logits, cap, vocab):
+    vocab = min(vocab, logits.size(-1))
+    if logits.is_cuda and logits.dtype == torch.bfloat16:
+        return _SoftcapLogitsFn.apply(logits, float(cap), vocab)
+    logits = logits[..., :vocab].float()
+    return cap * torch.tanh(logits / cap) if cap > 0 else logits
+
+
 def lm_head_logits_grad(x, w, cap, vocab, grad_acc=None, w_t=False):
     """Differentiable soft-capped fp32 logits (distillation / label-smoothing paths, unlimited/train.py:603-634)."""
-    logits = linear(x, w, grad_acc, w_t)[..., :vocab].float()
-    return cap * torch.tanh(logits / cap) if cap > 0 else logits
+    return _softcap_logits(linear(x, w, grad_acc, w_t), cap, vocab)
 
 
 def lm_head_logits(x, w, cap, vocab, w_t=False):
@@ -676,8 +710,48 @@ def lm_head_logits(x, w, cap, vocab, w_t=False):
         logits = gemm(x2, w, b_mn=w_t).view(*x.shape[:-1], -1)
     else:
         logits = (x @ w.to(x.dtype)) if w_t else F.linear(x, w.to(x.dtype))
-    logits = logits[..., :vocab].float()
-    return cap * torch.tanh(logits / cap) if cap > 0 else logits
+    return _softcap_logits(logits, cap, vocab)
+
+
+class _DistillFn(Function):
+    """(mean cross-entropy, mean KL(teacher / T || student / T)) over the rows whose target is not -1, fp32 logits [M, V]."""
+
+    @staticmethod
+    def forward(ctx, s, t, y, T, label_smoothing):
+        s, t, y = _c(s), _c(t), _c(y)
+        M, V = s.shape
+        rows = torch.empty((5, M), dtype=torch.float32, device=s.device)      # ce, kl, three log-sum-exps
+        _call("sr_distill_fwd", [c_void_p] * 6 + [c_long, c_int, c_float, c_float, c_void_p], s.data_ptr(), t.data_ptr(), y.data_ptr(),
+              rows[0].data_ptr(), rows[1].data_ptr(), rows[2].data_ptr(), M, V, T, label_smoothing, _lib.stream_ptr())
+        n = (y != -1).sum().float()
+        ctx.args = (T, label_smoothing)
+        ctx.save_for_backward(s, t, y, rows[2:], n)
+        return rows[0].sum() / n, rows[1].sum() / n
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, g_ce, g_kl):
+        s, t, y, stats, n = ctx.saved_tensors
+        T, label_smoothing = ctx.args
+        g_ce, g_kl = g_ce.float(), g_kl.float()
+        ds = torch.empty_like(s)
+        _call("sr_distill_bwd", [c_void_p] * 8 + [c_long, c_int, c_float, c_float, c_void_p], s.data_ptr(), t.data_ptr(), y.data_ptr(),
+              stats.data_ptr(), n.data_ptr(), g_ce.data_ptr(), g_kl.data_ptr(), ds.data_ptr(), s.size(0), s.size(1), T,
+              label_smoothing, _lib.stream_ptr())
+        return ds, None, None, None, None
+
+
+def distill_terms(s, t, y, T, label_smoothing=0.0):
+    """Cross-entropy and temperature-T KL terms of a distillation loss (unlimited/train.py:1631-1656): fp32 logits [M, V] of
+    student and teacher, targets [M] with -1 ignored. A teacher that itself needs a gradient takes the op-by-op form."""
+    if s.is_cuda and s.numel() > 0 and y.dtype == torch.int64 and s.shape == t.shape and \
+            not (torch.is_grad_enabled() and t.requires_grad):
+        return _DistillFn.apply(s, t, y, float(T), float(label_smoothing))
+    mask = y != -1
+    ce = F.cross_entropy(s, y, label_smoothing=label_smoothing, ignore_index=-1)
+    kl = F.kl_div(F.log_softmax(s[mask] / T, dim=-1), F.log_softmax(t[mask] / T, dim=-1), reduction="batchmean",
+                  log_target=True)
+    return ce, kl
 
 
 # =============================================================================== attention (train.py:211-213, 307)

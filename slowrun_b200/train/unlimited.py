@@ -20,7 +20,6 @@ from typing import Dict, List, Optional
 
 import torch
 import torch.distributed as dist
-import torch.nn.functional as F
 
 import copy
 import dataclasses
@@ -28,6 +27,7 @@ import dataclasses
 from ..config import TrainConfig
 from ..data.loader import EnsembleTokenLoader, TokenLoader
 from ..models.gpt import build_model
+from ..ops import functional as ops
 from ..optim.groups import build_param_groups
 from ..optim.muon_adamw import ShardedMuonAdamW
 from ..parallel.comm import DistInfo, TorchComm, init_distributed, print0
@@ -251,10 +251,8 @@ def distillation_loss(student_logits, teacher_logits, targets, mtp_loss, mtp_wei
     s = student_logits.reshape(-1, student_logits.size(-1)).float()
     t = teacher_logits.reshape(-1, teacher_logits.size(-1)).float()
     y = targets.reshape(-1)
-    mask = y != -1
-    ce = F.cross_entropy(s, y, label_smoothing=label_smoothing, ignore_index=-1)
-    kl = F.kl_div(F.log_softmax(s[mask] / T, dim=-1), F.log_softmax(t[mask] / T, dim=-1), reduction="batchmean",
-                  log_target=True) * (T ** 2)
+    ce, kl = ops.distill_terms(s, t, y, T, label_smoothing)
+    kl = kl * (T ** 2)
     normal = ce + (mtp_weight * mtp_loss if mtp_loss is not None else 0.0)
     return (1 - alpha) * normal + alpha * kl
 
