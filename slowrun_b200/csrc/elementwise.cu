@@ -15,6 +15,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 namespace {
 
 constexpr int kWarpsPerBlock = 8;
@@ -55,16 +57,18 @@ __device__ __forceinline__ float block_sum(float v, float* smem) {
   return r;  // valid in warp 0
 }
 
-// counter-based uniform in [0,1): one hash per element index, reproducible in backward
+// counter-based uniform in [0,1): one hash per element index, reproducible in backward. The element is kept when the upper 24
+// bits of the hash, as a fraction, are >= p: compared as integers against ceil(p 2^24) (exact, since p 2^24 is), which spares
+// a conversion and a product per element.
 __device__ __forceinline__ uint32_t mix32(uint64_t z) {
   z += 0x9E3779B97F4A7C15ull;
   z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
   z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
   return static_cast<uint32_t>((z ^ (z >> 31)) >> 32);
 }
-__device__ __forceinline__ bool keep_elem(uint64_t seed, uint64_t idx, float p) {
-  const uint32_t h = mix32(seed * 0x100000001B3ull + idx);
-  return (h >> 8) * (1.0f / 16777216.0f) >= p;
+__device__ __forceinline__ uint32_t keep_threshold(float p) { return static_cast<uint32_t>(ceilf(p * 16777216.f)); }
+__device__ __forceinline__ bool keep_elem(uint64_t seed, uint64_t idx, uint32_t threshold) {
+  return (mix32(seed * 0x100000001B3ull + idx) >> 8) >= threshold;
 }
 
 // ------------------------------------------------------------------ rmsnorm
@@ -505,13 +509,14 @@ __global__ void dropout_add_fwd_kernel(const __nv_bfloat16* __restrict__ x_mid, 
   const uint64_t seed = salt + (seed_ptr ? (*seed_ptr) * 0x9E3779B97F4A7C15ull : 0ull);
   const float keep = (x_in != nullptr) ? *keep_p : 1.f;
   const float scale = 1.f / (1.f - p);
+  const uint32_t thr = keep_threshold(p);
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (long)gridDim.x * blockDim.x) {
     float a[8], b[8], o[8];
     load8(x_mid + i * 8, a);
     load8(y + i * 8, b);
     if (p > 0.f) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) b[j] = keep_elem(seed, (uint64_t)i * 8 + j, p) ? b[j] * scale : 0.f;
+      for (int j = 0; j < 8; ++j) b[j] = keep_elem(seed, (uint64_t)i * 8 + j, thr) ? b[j] * scale : 0.f;
     }
     if (x_in != nullptr) {
       float xi[8];
@@ -533,12 +538,13 @@ __global__ void dropout_add_bwd_kernel(const __nv_bfloat16* __restrict__ g, cons
   const uint64_t seed = salt + (seed_ptr ? (*seed_ptr) * 0x9E3779B97F4A7C15ull : 0ull);
   const float keep = (keep_p != nullptr) ? *keep_p : 1.f;
   const float scale = 1.f / (1.f - p);
+  const uint32_t thr = keep_threshold(p);
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (long)gridDim.x * blockDim.x) {
     float gg[8], o[8];
     load8(g + i * 8, gg);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const bool k = (p > 0.f) ? keep_elem(seed, (uint64_t)i * 8 + j, p) : true;
+      const bool k = (p > 0.f) ? keep_elem(seed, (uint64_t)i * 8 + j, thr) : true;
       o[j] = k ? keep * scale * gg[j] : 0.f;
     }
     store8(dy + i * 8, o);
@@ -567,6 +573,7 @@ __global__ void add_norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const _
   const int lane = threadIdx.x & 31;
   const uint64_t seed = salt + (seed_ptr ? (*seed_ptr) * 0x9E3779B97F4A7C15ull : 0ull);
   const float scale = 1.f / (1.f - p);
+  const uint32_t thr = keep_threshold(p);
   const long base = row * (long)D;
   float ss = 0.f;
   for (int c = lane * 8; c < D; c += 256) {
@@ -575,7 +582,7 @@ __global__ void add_norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const _
     load8(y + base + c, b);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      if (p > 0.f) b[j] = keep_elem(seed, (uint64_t)(base + c + j), p) ? b[j] * scale : 0.f;
+      if (p > 0.f) b[j] = keep_elem(seed, (uint64_t)(base + c + j), thr) ? b[j] * scale : 0.f;
       a[j] = __bfloat162float(__float2bfloat16(a[j] + b[j]));
       ss += a[j] * a[j];
     }
@@ -603,6 +610,7 @@ __global__ void norm_bwd_drop_kernel(const __nv_bfloat16* __restrict__ x_mid, co
   const int lane = threadIdx.x & 31;
   const uint64_t seed = salt + (seed_ptr ? (*seed_ptr) * 0x9E3779B97F4A7C15ull : 0ull);
   const float scale = 1.f / (1.f - p);
+  const uint32_t thr = keep_threshold(p);
   const long base = row * (long)D;
   float ss = 0.f, dot = 0.f;
   for (int c = lane * 8; c < D; c += 256) {
@@ -627,11 +635,297 @@ __global__ void norm_bwd_drop_kernel(const __nv_bfloat16* __restrict__ x_mid, co
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       o[i] = __bfloat162float(__float2bfloat16(r * g[i] - k * f[i] + a[i]));
-      const bool keep = (p > 0.f) ? keep_elem(seed, (uint64_t)(base + c + i), p) : true;
+      const bool keep = (p > 0.f) ? keep_elem(seed, (uint64_t)(base + c + i), thr) : true;
       d[i] = keep ? scale * o[i] : 0.f;
     }
     store8(dx_mid + base + c, o);
     store8(dy + base + c, d);
+  }
+}
+
+// ------------------------------------------------------------------ the same four row kernels, a row held by a group of threads
+// The kernels above give a row to one warp, which walks it twice: at D = 2560 ten dependent steps of 16-byte loads per pass,
+// with 8192 rows filling less than one wave. Here TPR threads hold a row in registers (VPT vectors of 8 each): every load of
+// the row is in flight at once, each input is read once, and the only wait is the reduction over the group. Blocks walk over
+// rows, so the scalar sums of norm_bwd_mix cost three atomics per block and not per eight rows.
+// us, warp per row -> these, [8192, 2560]: norm_bwd_mix 110 -> 79, norm_bwd_drop 72 -> 64, mix_norm_fwd 48 -> 37, add_norm_fwd
+// 50 -> 46 (the dropout hash bounds the two with a mask); [65536, 1024]: 247 -> 226, 182 -> 158, 129 -> 98, 129 -> 127.
+constexpr int kRowThreads = 128;
+
+// sums of a and b over the TPR threads of a row; `red` holds 2 x 4 pairs that alternate, so one barrier per call suffices
+template <int TPR>
+__device__ __forceinline__ float2 group_sum(float a, float b, float2 (&red)[2][4], int& turn) {
+  a = warp_sum(a);
+  b = warp_sum(b);
+  const int warp = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0) red[turn][warp] = make_float2(a, b);
+  __syncthreads();
+  constexpr int W = TPR / 32;
+  const int w0 = warp / W * W;
+  float2 r = red[turn][w0];
+#pragma unroll
+  for (int i = 1; i < W; ++i) {
+    r.x += red[turn][w0 + i].x;
+    r.y += red[turn][w0 + i].y;
+  }
+  turn ^= 1;
+  return r;
+}
+__device__ __forceinline__ void unpack8(const uint4& t, float (&f)[8]) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&t);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 a = __bfloat1622float2(h[i]);
+    f[2 * i] = a.x;
+    f[2 * i + 1] = a.y;
+  }
+}
+__device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16(x)); }
+
+// f(row, valid) for the rows of this group; all threads of the block make the same number of steps
+#define SR_FOR_ROWS(TPR)                                                                                    \
+  constexpr int RPB = kRowThreads / (TPR);                                                                  \
+  const int tid = threadIdx.x % (TPR);                                                                      \
+  for (long row0 = (long)blockIdx.x * RPB; row0 < rows; row0 += (long)gridDim.x * RPB)
+
+template <int TPR, int VPT, typename F>
+__device__ __forceinline__ void row_vectors(int tid, int D, bool valid, F f) {
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int c = (tid + i * TPR) * 8;
+    if (valid && c < D) f(i, c);
+  }
+}
+#define LDV(p) (*reinterpret_cast<const uint4*>(p))
+
+template <int TPR, int VPT>
+__global__ void __launch_bounds__(kRowThreads)
+mix_norm_fwd_rows(const __nv_bfloat16* __restrict__ xp, const __nv_bfloat16* __restrict__ x0, const __nv_bfloat16* __restrict__ skip,
+                  __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ a_out, const float* __restrict__ lr_p,
+                  const float* __restrict__ l0_p, const float* __restrict__ ws_p, long rows, int D, float eps) {
+  __shared__ float2 red[2][4];
+  int turn = 0;
+  const float lr = *lr_p, l0 = *l0_p, ws = skip ? *ws_p : 0.f;
+  SR_FOR_ROWS(TPR) {
+    const long row = row0 + threadIdx.x / TPR;
+    const bool valid = row < rows;
+    const long base = row * (long)D;
+    uint4 A[VPT], B[VPT], S[VPT];
+    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
+      A[i] = LDV(xp + base + c);
+      B[i] = LDV(x0 + base + c);
+      if (skip) S[i] = LDV(skip + base + c);
+    });
+    float v[VPT][8];
+    float ss = 0.f;
+    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
+      float a[8], b[8], sk[8];
+      unpack8(A[i], a);
+      unpack8(B[i], b);
+      if (skip) {
+        unpack8(S[i], sk);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a[j] += ws * sk[j];
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        v[i][j] = round_bf16(lr * a[j] + l0 * b[j]);
+        ss += v[i][j] * v[i][j];
+      }
+      store8(x + base + c, v[i]);
+    });
+    const float r = rsqrtf(group_sum<TPR>(ss, 0.f, red, turn).x / D + eps);
+    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[i][j] *= r;
+      store8(a_out + base + c, v[i]);
+    });
+  }
+}
+
+template <int TPR, int VPT>
+__global__ void __launch_bounds__(kRowThreads)
+add_norm_fwd_rows(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ x_mid,
+                  __nv_bfloat16* __restrict__ n, long rows, int D, float eps, float p, uint64_t salt,
+                  const unsigned long long* __restrict__ seed_ptr) {
+  __shared__ float2 red[2][4];
+  int turn = 0;
+  const uint64_t seed = salt + (seed_ptr ? (*seed_ptr) * 0x9E3779B97F4A7C15ull : 0ull);
+  const float scale = 1.f / (1.f - p);
+  const uint32_t thr = keep_threshold(p);
+  SR_FOR_ROWS(TPR) {
+    const long row = row0 + threadIdx.x / TPR;
+    const bool valid = row < rows;
+    const long base = row * (long)D;
+    uint4 A[VPT], B[VPT];
+    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
+      A[i] = LDV(x + base + c);
+      B[i] = LDV(y + base + c);
+    });
+    float v[VPT][8];
+    float ss = 0.f;
+    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
+      float a[8], b[8];
+      unpack8(A[i], a);
+      unpack8(B[i], b);
+      if (p > 0.f) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) b[j] = keep_elem(seed, (uint64_t)(base + c + j), thr) ? b[j] * scale : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        v[i][j] = round_bf16(a[j] + b[j]);
+        ss += v[i][j] * v[i][j];
+      }
+      store8(x_mid + base + c, v[i]);
+    });
+    const float r = rsqrtf(group_sum<TPR>(ss, 0.f, red, turn).x / D + eps);
+    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[i][j] *= r;
+      store8(n + base + c, v[i]);
+    });
+  }
+}
+
+template <int TPR, int VPT>
+__global__ void __launch_bounds__(kRowThreads)
+norm_bwd_drop_rows(const __nv_bfloat16* __restrict__ x_mid, const __nv_bfloat16* __restrict__ dn, const __nv_bfloat16* __restrict__ g_res,
+                   __nv_bfloat16* __restrict__ dx_mid, __nv_bfloat16* __restrict__ dy, long rows, int D, float eps, float p,
+                   uint64_t salt, const unsigned long long* __restrict__ seed_ptr) {
+  __shared__ float2 red[2][4];
+  int turn = 0;
+  const uint64_t seed = salt + (seed_ptr ? (*seed_ptr) * 0x9E3779B97F4A7C15ull : 0ull);
+  const float scale = 1.f / (1.f - p);
+  const uint32_t thr = keep_threshold(p);
+  SR_FOR_ROWS(TPR) {
+    const long row = row0 + threadIdx.x / TPR;
+    const bool valid = row < rows;
+    const long base = row * (long)D;
+    uint4 X[VPT], G[VPT], R[VPT];
+    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
+      X[i] = LDV(x_mid + base + c);
+      G[i] = LDV(dn + base + c);
+      R[i] = LDV(g_res + base + c);
+    });
+    float ss = 0.f, dot = 0.f;
+    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int) {
+      float f[8], g[8];
+      unpack8(X[i], f);
+      unpack8(G[i], g);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        ss += f[j] * f[j];
+        dot += f[j] * g[j];
+      }
+    });
+    const float2 t = group_sum<TPR>(ss, dot, red, turn);
+    const float r = rsqrtf(t.x / D + eps);
+    const float k = r * r * r * t.y / D;
+    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
+      float f[8], g[8], a[8], o[8], d[8];
+      unpack8(X[i], f);
+      unpack8(G[i], g);
+      unpack8(R[i], a);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = round_bf16(r * g[j] - k * f[j] + a[j]);
+      store8(dx_mid + base + c, o);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const bool keep = (p > 0.f) ? keep_elem(seed, (uint64_t)(base + c + j), thr) : true;
+        d[j] = keep ? scale * o[j] : 0.f;
+      }
+      store8(dy + base + c, d);
+    });
+  }
+}
+
+template <int TPR, int VPT>
+__global__ void __launch_bounds__(kRowThreads)
+norm_bwd_mix_rows(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ da, const __nv_bfloat16* __restrict__ g_res,
+                  const __nv_bfloat16* __restrict__ g_res2, const __nv_bfloat16* __restrict__ xp, const __nv_bfloat16* __restrict__ x0,
+                  const __nv_bfloat16* __restrict__ skip, __nv_bfloat16* __restrict__ dxp, __nv_bfloat16* __restrict__ dx0,
+                  __nv_bfloat16* __restrict__ dskip, const float* __restrict__ lr_p, const float* __restrict__ l0_p,
+                  const float* __restrict__ ws_p, float* __restrict__ d_lr, float* __restrict__ d_l0, float* __restrict__ d_ws,
+                  long rows, int D, float eps) {
+  __shared__ float2 red[2][4];
+  __shared__ float red1[32];
+  int turn = 0;
+  const float lr = *lr_p, l0 = *l0_p, ws = skip ? *ws_p : 0.f;
+  float s_lr = 0.f, s_l0 = 0.f, s_ws = 0.f;
+  SR_FOR_ROWS(TPR) {
+    const long row = row0 + threadIdx.x / TPR;
+    const bool valid = row < rows;
+    const long base = row * (long)D;
+    uint4 X[VPT], G[VPT], R[VPT], R2[VPT], A[VPT], B[VPT], S[VPT];
+    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
+      X[i] = LDV(x + base + c);
+      G[i] = LDV(da + base + c);
+      R[i] = LDV(g_res + base + c);
+      if (g_res2) R2[i] = LDV(g_res2 + base + c);
+      A[i] = LDV(xp + base + c);
+      B[i] = LDV(x0 + base + c);
+      if (skip) S[i] = LDV(skip + base + c);
+    });
+    float ss = 0.f, dot = 0.f;
+    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int) {
+      float f[8], g[8];
+      unpack8(X[i], f);
+      unpack8(G[i], g);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        ss += f[j] * f[j];
+        dot += f[j] * g[j];
+      }
+    });
+    const float2 t = group_sum<TPR>(ss, dot, red, turn);
+    const float r = rsqrtf(t.x / D + eps);
+    const float k = r * r * r * t.y / D;
+    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
+      float f[8], g[8], e[8], a[8], b[8], o[8];
+      unpack8(X[i], f);
+      unpack8(G[i], g);
+      unpack8(R[i], e);
+      if (g_res2) {   // second residual gradient (the stochastic-depth bypass), added in bf16 like a separate add would
+        float e2[8];
+        unpack8(R2[i], e2);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) e[j] = round_bf16(e[j] + e2[j]);
+      }
+      unpack8(A[i], a);
+      unpack8(B[i], b);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) g[j] = round_bf16(r * g[j] - k * f[j] + e[j]);
+      if (skip) {
+        float sk[8];
+        unpack8(S[i], sk);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          a[j] += ws * sk[j];
+          s_ws += g[j] * lr * sk[j];
+          o[j] = lr * ws * g[j];
+        }
+        store8(dskip + base + c, o);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        s_lr += g[j] * a[j];
+        s_l0 += g[j] * b[j];
+        o[j] = lr * g[j];
+      }
+      store8(dxp + base + c, o);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = l0 * g[j];
+      store8(dx0 + base + c, o);
+    });
+  }
+  s_lr = block_sum(s_lr, red1);
+  s_l0 = block_sum(s_l0, red1);
+  s_ws = block_sum(s_ws, red1);
+  if (threadIdx.x == 0) {
+    atomicAdd(d_lr, s_lr);
+    atomicAdd(d_l0, s_l0);
+    if (skip) atomicAdd(d_ws, s_ws);
   }
 }
 
@@ -664,6 +958,23 @@ inline int grid_for(long n, int per_block) {
   return (int)(b < 1 ? 1 : (b > cap ? cap : b));
 }
 inline int rc() { return cudaGetLastError() == cudaSuccess ? 0 : -5; }
+
+// Rows of 264 to 4096 elements go to the *_rows kernels: 64 threads up to 512, 128 beyond, as many vectors per thread as the
+// row needs. Shorter rows are one step for a warp as it is, longer ones would not fit the registers.
+template <typename F>
+bool row_dispatch(int D, F f) {
+  if (D <= 256 || D > 4096) return false;
+  if (D <= 512) f(std::integral_constant<int, 64>(), std::integral_constant<int, 1>());
+  else if (D <= 1024) f(std::integral_constant<int, 128>(), std::integral_constant<int, 1>());
+  else if (D <= 2048) f(std::integral_constant<int, 128>(), std::integral_constant<int, 2>());
+  else if (D <= 3072) f(std::integral_constant<int, 128>(), std::integral_constant<int, 3>());
+  else f(std::integral_constant<int, 128>(), std::integral_constant<int, 4>());
+  return true;
+}
+inline unsigned row_grid(long rows, int tpr, int blocks_per_sm) {
+  const long b = (rows * tpr + kRowThreads - 1) / kRowThreads, cap = (long)sm_count() * blocks_per_sm;
+  return (unsigned)(b < cap ? b : cap);
+}
 
 }  // namespace
 
@@ -767,6 +1078,11 @@ extern "C" int sr_add_norm_fwd(const void* x, const void* y, void* x_mid, void* 
                                unsigned long long seed, const unsigned long long* seed_ptr, cudaStream_t s) {
   if (D % 8) return -2;
   if (rows <= 0) return 0;
+  if (row_dispatch(D, [&](auto tpr, auto vpt) {
+        add_norm_fwd_rows<tpr.value, vpt.value><<<row_grid(rows, tpr.value, 64), kRowThreads, 0, s>>>(
+            BF(x), BF(y), BFM(x_mid), BFM(n), rows, D, eps, p, seed, seed_ptr);
+      }))
+    return rc();
   add_norm_fwd_kernel<<<(unsigned)((rows + kWarpsPerBlock - 1) / kWarpsPerBlock), kThreads, 0, s>>>(
       BF(x), BF(y), BFM(x_mid), BFM(n), rows, D, eps, p, seed, seed_ptr);
   return rc();
@@ -777,6 +1093,11 @@ extern "C" int sr_norm_bwd_drop(const void* x_mid, const void* dn, const void* g
                                 cudaStream_t s) {
   if (D % 8) return -2;
   if (rows <= 0) return 0;
+  if (row_dispatch(D, [&](auto tpr, auto vpt) {
+        norm_bwd_drop_rows<tpr.value, vpt.value><<<row_grid(rows, tpr.value, 64), kRowThreads, 0, s>>>(
+            BF(x_mid), BF(dn), BF(g_res), BFM(dx_mid), BFM(dy), rows, D, eps, p, seed, seed_ptr);
+      }))
+    return rc();
   norm_bwd_drop_kernel<<<(unsigned)((rows + kWarpsPerBlock - 1) / kWarpsPerBlock), kThreads, 0, s>>>(
       BF(x_mid), BF(dn), BF(g_res), BFM(dx_mid), BFM(dy), rows, D, eps, p, seed, seed_ptr);
   return rc();
@@ -787,6 +1108,11 @@ extern "C" int sr_mix_norm_fwd(const void* xp, const void* x0, const void* skip,
                                const float* l0, const float* ws, long rows, int D, float eps, cudaStream_t s) {
   if (D % 8) return -2;
   if (rows <= 0) return 0;
+  if (row_dispatch(D, [&](auto tpr, auto vpt) {
+        mix_norm_fwd_rows<tpr.value, vpt.value><<<row_grid(rows, tpr.value, 64), kRowThreads, 0, s>>>(
+            BF(xp), BF(x0), BF(skip), BFM(x), BFM(a), lr, l0, ws, rows, D, eps);
+      }))
+    return rc();
   mix_norm_fwd_kernel<<<(unsigned)((rows + kWarpsPerBlock - 1) / kWarpsPerBlock), kThreads, 0, s>>>(
       BF(xp), BF(x0), BF(skip), BFM(x), BFM(a), lr, l0, ws, rows, D, eps);
   return rc();
@@ -801,6 +1127,12 @@ extern "C" int sr_norm_bwd_mix(const void* x, const void* da, const void* g_res,
                                cudaStream_t s) {
   if (D % 8) return -2;
   if (rows <= 0) return 0;
+  if (row_dispatch(D, [&](auto tpr, auto vpt) {
+        norm_bwd_mix_rows<tpr.value, vpt.value><<<row_grid(rows, tpr.value, 8), kRowThreads, 0, s>>>(
+            BF(x), BF(da), BF(g_res), BF(g_res2), BF(xp), BF(x0), BF(skip), BFM(dxp), BFM(dx0), BFM(dskip), lr, l0, ws, d_lr,
+            d_l0, d_ws, rows, D, eps);
+      }))
+    return rc();
   norm_bwd_mix_kernel<<<(unsigned)((rows + kWarpsPerBlock - 1) / kWarpsPerBlock), kThreads, 0, s>>>(
       BF(x), BF(da), BF(g_res), BF(g_res2), BF(xp), BF(x0), BF(skip), BFM(dxp), BFM(dx0), BFM(dskip), lr, l0, ws, d_lr, d_l0, d_ws, rows, D, eps);
   return rc();
