@@ -20,6 +20,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <initializer_list>
+
 namespace {
 
 constexpr int kWarpsPerBlock = 8;
@@ -35,11 +37,6 @@ inline int sm_count() {
   return n;
 }
 
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
 __device__ __forceinline__ float2 ld2(const __nv_bfloat16* p) {
   return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
 }
@@ -47,239 +44,309 @@ __device__ __forceinline__ void st2(__nv_bfloat16* p, float a, float b) {
   *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b);
 }
 
-// ---------------------------------------------------------------------------------------------- qkv prep
-// One warp per (token, head); lane l owns elements {2l, 2l+1} and {64+2l, 64+2l+1} of each 128-wide head vector.
-__global__ void qkv_prep_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ ve,
-                                    const float* __restrict__ gate, const __nv_bfloat16* __restrict__ cosb,
-                                    const __nv_bfloat16* __restrict__ sinb, __nv_bfloat16* __restrict__ q_out,
-                                    __nv_bfloat16* __restrict__ k_out, __nv_bfloat16* __restrict__ v_out, long tokens, int H,
-                                    int T, float eps, int key_offset) {
-  const long wid = (long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-  if (wid >= tokens * H) return;
-  const int lane = threadIdx.x & 31;
-  const long tok = wid / H;
-  const int h = (int)(wid - tok * H);
-  const int t = (int)(tok % T);
-  const long d = (long)H * 128;
-  const float2 c = ld2(cosb + (long)t * 64 + 2 * lane);
-  const float2 s = ld2(sinb + (long)t * 64 + 2 * lane);
+// ---------------------------------------------------------------------------------------------- per-head vectors
+// The kernels below work on (token, head) vectors of 128 elements. Eight lanes hold one: lane l has elements 8l .. 8l+7 and
+// 64+8l .. 64+8l+7, i.e. both partners of its rotary pairs, in two 16-byte accesses per tensor. A warp then has four vectors
+// in flight and a reduction is three shuffles; with a warp per vector it was five shuffles and 4-byte accesses for one, and
+// the kernels were bound by instructions. us, warp per vector -> this, [8192, 20 heads]: qkv_prep fwd 76 -> 50, bwd 114 -> 86,
+// attn_post bwd 57 -> 37; [65536, 8 heads]: 217 -> 152, 342 -> 293, 272 -> 195, attn_post fwd 101 -> 65.
+constexpr int kVecPerBlock = kThreads / 8;
+
+struct Vec {
+  float lo[8], hi[8];
+};
+__device__ __forceinline__ void unpack8(const uint4& t, float (&f)[8]) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&t);
 #pragma unroll
-  for (int which = 0; which < 2; ++which) {
-    const __nv_bfloat16* p = qkv + tok * 3 * d + which * d + h * 128;
-    const float2 x1 = ld2(p + 2 * lane), x2 = ld2(p + 64 + 2 * lane);
-    float2 o1, o2;
-    o1.x = x1.x * c.x + x2.x * s.x;
-    o1.y = x1.y * c.y + x2.y * s.y;
-    o2.x = -x1.x * s.x + x2.x * c.x;
-    o2.y = -x1.y * s.y + x2.y * c.y;
-    float ss = o1.x * o1.x + o1.y * o1.y + o2.x * o2.x + o2.y * o2.y;
-    ss = warp_sum(ss);
-    const float r = rsqrtf(ss * (1.f / 128.f) + eps);
-    __nv_bfloat16* o = (which == 0 ? q_out : k_out) + wid * 128;
-    st2(o + 2 * lane, o1.x * r, o1.y * r);
-    if (which == 1 && key_offset) {
-      // upper half goes to the next token of the sequence (same head: H rows further); token 0 also keeps its own
-      if (t + 1 < T) st2(o + (long)H * 128 + 64 + 2 * lane, o2.x * r, o2.y * r);
-      if (t == 0) st2(o + 64 + 2 * lane, o2.x * r, o2.y * r);
-    } else {
-      st2(o + 64 + 2 * lane, o2.x * r, o2.y * r);
-    }
-  }
-  {
-    const __nv_bfloat16* p = qkv + tok * 3 * d + 2 * d + h * 128 + lane * 4;
-    float2 a0 = ld2(p), a1 = ld2(p + 2);
-    if (ve != nullptr) {
-      const float g = gate[wid];
-      const __nv_bfloat16* e = ve + tok * d + h * 128 + lane * 4;
-      const float2 e0 = ld2(e), e1 = ld2(e + 2);
-      a0.x += g * e0.x; a0.y += g * e0.y; a1.x += g * e1.x; a1.y += g * e1.y;
-    }
-    __nv_bfloat16* o = v_out + wid * 128 + lane * 4;
-    st2(o, a0.x, a0.y);
-    st2(o + 2, a1.x, a1.y);
+  for (int i = 0; i < 4; ++i) {
+    const float2 a = __bfloat1622float2(h[i]);
+    f[2 * i] = a.x;
+    f[2 * i + 1] = a.y;
   }
 }
+__device__ __forceinline__ void ld8(const __nv_bfloat16* p, float (&f)[8]) { unpack8(*reinterpret_cast<const uint4*>(p), f); }
+__device__ __forceinline__ void st8(__nv_bfloat16* p, const float (&f)[8]) {
+  uint4 t;
+  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&t);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+  *reinterpret_cast<uint4*>(p) = t;
+}
+__device__ __forceinline__ void ldf8(const float* p, float (&f)[8]) {
+  const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+  f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
+  f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+}
+// p: first element of the vector; l: lane within the eight
+__device__ __forceinline__ Vec ldv(const __nv_bfloat16* p, int l) {
+  Vec v;
+  ld8(p + 8 * l, v.lo);
+  ld8(p + 64 + 8 * l, v.hi);
+  return v;
+}
+__device__ __forceinline__ void stv(__nv_bfloat16* p, int l, const Vec& v) {
+  st8(p + 8 * l, v.lo);
+  st8(p + 64 + 8 * l, v.hi);
+}
+__device__ __forceinline__ float dot(const Vec& a, const Vec& b) {
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) s += a.lo[i] * b.lo[i] + a.hi[i] * b.hi[i];
+  return s;
+}
+// sum over the eight lanes of a vector
+__device__ __forceinline__ float sum8(float v) {
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
 
-__global__ void qkv_prep_bwd_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ ve,
-                                    const float* __restrict__ gate, const __nv_bfloat16* __restrict__ cosb,
-                                    const __nv_bfloat16* __restrict__ sinb, const __nv_bfloat16* __restrict__ dq,
-                                    const __nv_bfloat16* __restrict__ dk, const __nv_bfloat16* __restrict__ dv,
-                                    __nv_bfloat16* __restrict__ dqkv, __nv_bfloat16* __restrict__ dve,
-                                    float* __restrict__ dgate, long tokens, int H, int T, float eps,
-                                    const float* __restrict__ dq_f32, int key_offset,
-                                    const __nv_bfloat16* __restrict__ dv_extra) {
-  const long wid = (long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-  if (wid >= tokens * H) return;
-  const int lane = threadIdx.x & 31;
-  const long tok = wid / H;
-  const int h = (int)(wid - tok * H);
-  const int t = (int)(tok % T);
+// ---------------------------------------------------------------------------------------------- qkv prep
+__global__ void __launch_bounds__(kThreads)
+qkv_prep_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ ve, const float* __restrict__ gate,
+                    const __nv_bfloat16* __restrict__ cosb, const __nv_bfloat16* __restrict__ sinb, __nv_bfloat16* __restrict__ q_out,
+                    __nv_bfloat16* __restrict__ k_out, __nv_bfloat16* __restrict__ v_out, unsigned n, unsigned H, unsigned T, float eps,
+                    int key_offset) {
+  const unsigned id = blockIdx.x * kVecPerBlock + (threadIdx.x >> 3);
+  const bool valid = id < n;                      // the shuffles below want whole warps
+  const unsigned vid = valid ? id : n - 1;
+  const int l = threadIdx.x & 7;
+  const unsigned tok = vid / H, h = vid - tok * H, t = tok % T;
   const long d = (long)H * 128;
-  const float2 c = ld2(cosb + (long)t * 64 + 2 * lane);
-  const float2 s = ld2(sinb + (long)t * 64 + 2 * lane);
+  const __nv_bfloat16* in = qkv + (long)tok * 3 * d + h * 128;
+  float c[8], s[8];
+  ld8(cosb + (long)t * 64 + 8 * l, c);
+  ld8(sinb + (long)t * 64 + 8 * l, s);
+  const Vec x[2] = {ldv(in, l), ldv(in + d, l)};
+  Vec v = ldv(in + 2 * d, l);
+  if (ve != nullptr) {
+    const float g = gate[vid];
+    const Vec e = ldv(ve + (long)tok * d + h * 128, l);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      v.lo[i] += g * e.lo[i];
+      v.hi[i] += g * e.hi[i];
+    }
+  }
 #pragma unroll
   for (int which = 0; which < 2; ++which) {
-    const __nv_bfloat16* p = qkv + tok * 3 * d + which * d + h * 128;
-    const float2 x1 = ld2(p + 2 * lane), x2 = ld2(p + 64 + 2 * lane);
-    float2 o1, o2;
-    o1.x = x1.x * c.x + x2.x * s.x;
-    o1.y = x1.y * c.y + x2.y * s.y;
-    o2.x = -x1.x * s.x + x2.x * c.x;
-    o2.y = -x1.y * s.y + x2.y * c.y;
-    float2 g1, g2;
-    if (which == 0 && dq_f32 != nullptr) {   // dQ straight from the attention kernel's fp32 accumulator
-      const float* gp = dq_f32 + wid * 128;
-      g1 = *reinterpret_cast<const float2*>(gp + 2 * lane);
-      g2 = *reinterpret_cast<const float2*>(gp + 64 + 2 * lane);
-    } else {
-      const __nv_bfloat16* gp = (which == 0 ? dq : dk) + wid * 128;
-      g1 = ld2(gp + 2 * lane);
+    Vec o;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      o.lo[i] = x[which].lo[i] * c[i] + x[which].hi[i] * s[i];
+      o.hi[i] = -x[which].lo[i] * s[i] + x[which].hi[i] * c[i];
+    }
+    const float r = rsqrtf(sum8(dot(o, o)) * (1.f / 128.f) + eps);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      o.lo[i] *= r;
+      o.hi[i] *= r;
+    }
+    if (valid) {
+      __nv_bfloat16* p = (which == 0 ? q_out : k_out) + (long)vid * 128;
+      st8(p + 8 * l, o.lo);
       if (which == 1 && key_offset) {
-        // the upper half computed here was consumed by the next token (and by token 0 itself)
-        g2 = make_float2(0.f, 0.f);
-        if (t + 1 < T) g2 = ld2(gp + (long)H * 128 + 64 + 2 * lane);
-        if (t == 0) {
-          const float2 own = ld2(gp + 64 + 2 * lane);
-          g2.x += own.x;
-          g2.y += own.y;
-        }
+        // upper half goes to the next token of the sequence (same head: H vectors further); token 0 also keeps its own
+        if (t + 1 < T) st8(p + d + 64 + 8 * l, o.hi);
+        if (t == 0) st8(p + 64 + 8 * l, o.hi);
       } else {
-        g2 = ld2(gp + 64 + 2 * lane);
+        st8(p + 64 + 8 * l, o.hi);
       }
     }
-    float ss = o1.x * o1.x + o1.y * o1.y + o2.x * o2.x + o2.y * o2.y;
-    float dot = o1.x * g1.x + o1.y * g1.y + o2.x * g2.x + o2.y * g2.y;
-    ss = warp_sum(ss);
-    dot = warp_sum(dot);
-    const float r = rsqrtf(ss * (1.f / 128.f) + eps);
-    const float k = r * r * r * dot * (1.f / 128.f);
-    float2 d1, d2;
-    d1.x = r * g1.x - k * o1.x;
-    d1.y = r * g1.y - k * o1.y;
-    d2.x = r * g2.x - k * o2.x;
-    d2.y = r * g2.y - k * o2.y;
-    __nv_bfloat16* o = dqkv + tok * 3 * d + which * d + h * 128;
-    st2(o + 2 * lane, d1.x * c.x - d2.x * s.x, d1.y * c.y - d2.y * s.y);
-    st2(o + 64 + 2 * lane, d1.x * s.x + d2.x * c.x, d1.y * s.y + d2.y * c.y);
   }
-  {
-    const __nv_bfloat16* gp = dv + wid * 128 + lane * 4;
-    float2 g0 = ld2(gp), g1 = ld2(gp + 2);
-    if (dv_extra != nullptr) {    // second consumer of v (exclusive self-attention)
-      const float2 x0 = ld2(dv_extra + wid * 128 + lane * 4), x1 = ld2(dv_extra + wid * 128 + lane * 4 + 2);
-      g0.x += x0.x; g0.y += x0.y; g1.x += x1.x; g1.y += x1.y;
+  if (valid) stv(v_out + (long)vid * 128, l, v);
+}
+
+__global__ void __launch_bounds__(kThreads)
+qkv_prep_bwd_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ ve, const float* __restrict__ gate,
+                    const __nv_bfloat16* __restrict__ cosb, const __nv_bfloat16* __restrict__ sinb, const __nv_bfloat16* __restrict__ dq,
+                    const __nv_bfloat16* __restrict__ dk, const __nv_bfloat16* __restrict__ dv, __nv_bfloat16* __restrict__ dqkv,
+                    __nv_bfloat16* __restrict__ dve, float* __restrict__ dgate, unsigned n, unsigned H, unsigned T, float eps,
+                    const float* __restrict__ dq_f32, int key_offset, const __nv_bfloat16* __restrict__ dv_extra) {
+  const unsigned id = blockIdx.x * kVecPerBlock + (threadIdx.x >> 3);
+  const bool valid = id < n;
+  const unsigned vid = valid ? id : n - 1;
+  const int l = threadIdx.x & 7;
+  const unsigned tok = vid / H, h = vid - tok * H, t = tok % T;
+  const long d = (long)H * 128, at = (long)vid * 128;
+  const __nv_bfloat16* in = qkv + (long)tok * 3 * d + h * 128;
+  __nv_bfloat16* out = dqkv + (long)tok * 3 * d + h * 128;
+  float c[8], s[8];
+  ld8(cosb + (long)t * 64 + 8 * l, c);
+  ld8(sinb + (long)t * 64 + 8 * l, s);
+#pragma unroll
+  for (int which = 0; which < 2; ++which) {
+    const Vec x = ldv(in + which * d, l);
+    Vec g;
+    if (which == 0 && dq_f32 != nullptr) {   // dQ straight from the attention kernel's fp32 accumulator
+      ldf8(dq_f32 + at + 8 * l, g.lo);
+      ldf8(dq_f32 + at + 64 + 8 * l, g.hi);
+    } else {
+      const __nv_bfloat16* gp = (which == 0 ? dq : dk) + at;
+      ld8(gp + 8 * l, g.lo);
+      if (which == 1 && key_offset) {
+        // the upper half computed here was consumed by the next token (and by token 0 itself)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) g.hi[i] = 0.f;
+        if (t + 1 < T) ld8(gp + d + 64 + 8 * l, g.hi);
+        if (t == 0) {
+          float own[8];
+          ld8(gp + 64 + 8 * l, own);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) g.hi[i] += own[i];
+        }
+      } else {
+        ld8(gp + 64 + 8 * l, g.hi);
+      }
     }
-    __nv_bfloat16* o = dqkv + tok * 3 * d + 2 * d + h * 128 + lane * 4;
-    st2(o, g0.x, g0.y);
-    st2(o + 2, g1.x, g1.y);
-    if (ve != nullptr) {
-      const float g = gate[wid];
-      const __nv_bfloat16* e = ve + tok * d + h * 128 + lane * 4;
-      const float2 e0 = ld2(e), e1 = ld2(e + 2);
-      float dot = g0.x * e0.x + g0.y * e0.y + g1.x * e1.x + g1.y * e1.y;
-      dot = warp_sum(dot);
-      if (lane == 0) dgate[wid] = dot;
-      __nv_bfloat16* de = dve + tok * d + h * 128 + lane * 4;
-      st2(de, g * g0.x, g * g0.y);
-      st2(de + 2, g * g1.x, g * g1.y);
+    Vec o;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      o.lo[i] = x.lo[i] * c[i] + x.hi[i] * s[i];
+      o.hi[i] = -x.lo[i] * s[i] + x.hi[i] * c[i];
+    }
+    const float r = rsqrtf(sum8(dot(o, o)) * (1.f / 128.f) + eps);
+    const float k = r * r * r * sum8(dot(o, g)) * (1.f / 128.f);
+    Vec w;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float d1 = r * g.lo[i] - k * o.lo[i], d2 = r * g.hi[i] - k * o.hi[i];
+      w.lo[i] = d1 * c[i] - d2 * s[i];
+      w.hi[i] = d1 * s[i] + d2 * c[i];
+    }
+    if (valid) stv(out + which * d, l, w);
+  }
+  Vec g = ldv(dv + at, l);
+  if (dv_extra != nullptr) {    // second consumer of v (exclusive self-attention)
+    const Vec x = ldv(dv_extra + at, l);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      g.lo[i] += x.lo[i];
+      g.hi[i] += x.hi[i];
+    }
+  }
+  if (valid) stv(out + 2 * d, l, g);
+  if (ve != nullptr) {
+    const float gt = gate[vid];
+    const Vec e = ldv(ve + (long)tok * d + h * 128, l);
+    const float dg = sum8(dot(g, e));
+    if (valid) {
+      if (l == 0) dgate[vid] = dg;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        g.lo[i] *= gt;
+        g.hi[i] *= gt;
+      }
+      stv(dve + (long)tok * d + h * 128, l, g);
     }
   }
 }
 
 // ---------------------------------------------------------------------------------------------- after attention
-// One warp per (token, head) row of 128; lane l owns elements 4l .. 4l+3. alpha: fp32 [H] (raw, tanh applied here) or
-// null = no exclusive self-attention.
-struct Row4 {
-  float v[4];
-};
-__device__ __forceinline__ Row4 ld4(const __nv_bfloat16* p) {
-  const float2 a = ld2(p), b = ld2(p + 2);
-  return Row4{{a.x, a.y, b.x, b.y}};
-}
-__device__ __forceinline__ float dot4(const Row4& a, const Row4& b) {
-  return a.v[0] * b.v[0] + a.v[1] * b.v[1] + a.v[2] * b.v[2] + a.v[3] * b.v[3];
-}
-
-__global__ void attn_post_fwd_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ v,
-                                     const float* __restrict__ gate, const float* __restrict__ alpha,
-                                     __nv_bfloat16* __restrict__ out, long rows, int H, float xsa_eps) {
-  const int lane = threadIdx.x & 31;
-  for (long wid = (long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); wid < rows; wid += (long)gridDim.x * kWarpsPerBlock) {
-    Row4 yy = ld4(y + wid * 128 + lane * 4);
+// alpha: fp32 [H] (raw, tanh applied here) or null = no exclusive self-attention.
+__global__ void __launch_bounds__(kThreads)
+attn_post_fwd_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ v, const float* __restrict__ gate,
+                     const float* __restrict__ alpha, __nv_bfloat16* __restrict__ out, unsigned n, unsigned H, float xsa_eps) {
+  const int l = threadIdx.x & 7;
+  const unsigned steps = (n + gridDim.x * kVecPerBlock - 1) / (gridDim.x * kVecPerBlock);
+  for (unsigned it = 0; it < steps; ++it) {
+    const unsigned id = (it * gridDim.x + blockIdx.x) * kVecPerBlock + (threadIdx.x >> 3);
+    const bool valid = id < n;
+    const unsigned vid = valid ? id : n - 1;
+    const long at = (long)vid * 128;
+    Vec yy = ldv(y + at, l);
+    const float s = gate[vid];
     if (alpha != nullptr) {
-      const Row4 vv = ld4(v + wid * 128 + lane * 4);
-      const float n = fmaxf(sqrtf(warp_sum(dot4(vv, vv))), xsa_eps);
-      const float c = warp_sum(dot4(yy, vv)) / n;
-      const float k = tanhf(alpha[wid % H]) * c / n;
+      const Vec vv = ldv(v + at, l);
+      const float nn = fmaxf(sqrtf(sum8(dot(vv, vv))), xsa_eps);
+      const float c = sum8(dot(yy, vv)) / nn;
+      const float k = tanhf(alpha[vid % H]) * c / nn;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) yy.v[i] -= k * vv.v[i];
+      for (int i = 0; i < 8; ++i) {
+        yy.lo[i] -= k * vv.lo[i];
+        yy.hi[i] -= k * vv.hi[i];
+      }
     }
-    const float s = gate[wid];
-    __nv_bfloat16* o = out + wid * 128 + lane * 4;
-    st2(o, yy.v[0] * s, yy.v[1] * s);
-    st2(o + 2, yy.v[2] * s, yy.v[3] * s);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      yy.lo[i] *= s;
+      yy.hi[i] *= s;
+    }
+    if (valid) stv(out + at, l, yy);
   }
 }
 
 // g: gradient of the gated output. Writes dy (gradient of the attention output), dgate (w.r.t. the gate value),
 // delta[b, h, t] = sum_d dy * y, and with alpha: dv_x (this op's gradient of v) and dalpha[H] += (atomics, one per
 // block and head).
-__global__ void attn_post_bwd_kernel(const __nv_bfloat16* __restrict__ g, const __nv_bfloat16* __restrict__ y,
-                                     const __nv_bfloat16* __restrict__ v, const float* __restrict__ gate,
-                                     const float* __restrict__ alpha, __nv_bfloat16* __restrict__ dy,
-                                     float* __restrict__ dgate, float* __restrict__ delta,
-                                     __nv_bfloat16* __restrict__ dv_x, float* __restrict__ dalpha, long rows, int H, int T,
-                                     float xsa_eps) {
+__global__ void __launch_bounds__(kThreads)
+attn_post_bwd_kernel(const __nv_bfloat16* __restrict__ g, const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ v,
+                     const float* __restrict__ gate, const float* __restrict__ alpha, __nv_bfloat16* __restrict__ dy,
+                     float* __restrict__ dgate, float* __restrict__ delta, __nv_bfloat16* __restrict__ dv_x, float* __restrict__ dalpha,
+                     unsigned n, unsigned H, unsigned T, float xsa_eps) {
   __shared__ float dal[64];
-  const int lane = threadIdx.x & 31;
+  const int l = threadIdx.x & 7;
   if (alpha != nullptr) {
     if (threadIdx.x < 64) dal[threadIdx.x] = 0.f;
     __syncthreads();
   }
-  for (long wid = (long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); wid < rows; wid += (long)gridDim.x * kWarpsPerBlock) {
-    const long tok = wid / H;
-    const int h = (int)(wid - tok * H);
-    const Row4 gg = ld4(g + wid * 128 + lane * 4);
-    const Row4 yy = ld4(y + wid * 128 + lane * 4);
-    const float s = gate[wid];
-    Row4 d;      // gradient of the attention output
+  const unsigned steps = (n + gridDim.x * kVecPerBlock - 1) / (gridDim.x * kVecPerBlock);
+  for (unsigned it = 0; it < steps; ++it) {
+    const unsigned id = (it * gridDim.x + blockIdx.x) * kVecPerBlock + (threadIdx.x >> 3);
+    const bool valid = id < n;
+    const unsigned vid = valid ? id : n - 1;
+    const unsigned tok = vid / H, h = vid - tok * H;
+    const long at = (long)vid * 128;
+    const Vec gg = ldv(g + at, l), yy = ldv(y + at, l);
+    const float s = gate[vid];
+    Vec d;       // gradient of the attention output
     float dg;    // sum_d g * (output before the gate)
     if (alpha != nullptr) {
-      const Row4 vv = ld4(v + wid * 128 + lane * 4);
-      const float nrm = sqrtf(warp_sum(dot4(vv, vv)));
-      const float n = fmaxf(nrm, xsa_eps);
-      const float inv = 1.f / n;
-      const float c = warp_sum(dot4(yy, vv)) * inv;          // y . u,  u = v / n
+      const Vec vv = ldv(v + at, l);
+      const float nrm = sqrtf(sum8(dot(vv, vv)));
+      const float inv = 1.f / fmaxf(nrm, xsa_eps);
+      const float c = sum8(dot(yy, vv)) * inv;                // y . u,  u = v / max(|v|, eps)
       const float a = tanhf(alpha[h]);
-      const float gy = warp_sum(dot4(gg, yy)), gu = warp_sum(dot4(gg, vv)) * inv;
+      const float gy = sum8(dot(gg, yy)), gu = sum8(dot(gg, vv)) * inv;
       dg = gy - a * c * gu;                                   // g . (y - a c u)
       const float p = s * gu;                                 // (s g) . u
-      Row4 du;
+      Vec du;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float u = vv.v[i] * inv, dyp = s * gg.v[i];
-        d.v[i] = dyp - a * p * u;
-        du.v[i] = -a * (p * yy.v[i] + c * dyp);
+      for (int i = 0; i < 8; ++i) {
+        const float d0 = s * gg.lo[i], d1 = s * gg.hi[i];
+        d.lo[i] = d0 - a * p * (vv.lo[i] * inv);
+        d.hi[i] = d1 - a * p * (vv.hi[i] * inv);
+        du.lo[i] = -a * (p * yy.lo[i] + c * d0);
+        du.hi[i] = -a * (p * yy.hi[i] + c * d1);
       }
       // v -> u = v / max(|v|, eps): the projection term only where the norm is not clamped
-      const float duu = nrm > xsa_eps ? warp_sum(dot4(du, vv)) * inv : 0.f;
-      __nv_bfloat16* o = dv_x + wid * 128 + lane * 4;
-      st2(o, (du.v[0] - duu * vv.v[0] * inv) * inv, (du.v[1] - duu * vv.v[1] * inv) * inv);
-      st2(o + 2, (du.v[2] - duu * vv.v[2] * inv) * inv, (du.v[3] - duu * vv.v[3] * inv) * inv);
-      if (lane == 0) atomicAdd(&dal[h], -c * p * (1.f - a * a));
-    } else {
-      dg = warp_sum(dot4(gg, yy));
+      const float proj = sum8(dot(du, vv)) * inv;
+      const float duu = nrm > xsa_eps ? proj : 0.f;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) d.v[i] = s * gg.v[i];
+      for (int i = 0; i < 8; ++i) {
+        du.lo[i] = (du.lo[i] - duu * vv.lo[i] * inv) * inv;
+        du.hi[i] = (du.hi[i] - duu * vv.hi[i] * inv) * inv;
+      }
+      if (valid) {
+        stv(dv_x + at, l, du);
+        if (l == 0) atomicAdd(&dal[h], -c * p * (1.f - a * a));
+      }
+    } else {
+      dg = sum8(dot(gg, yy));
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        d.lo[i] = s * gg.lo[i];
+        d.hi[i] = s * gg.hi[i];
+      }
     }
-    const float dl = warp_sum(dot4(d, yy));
-    if (lane == 0) {
-      dgate[wid] = dg;
-      delta[((tok / T) * H + h) * T + (tok % T)] = dl;
+    const float dl = sum8(dot(d, yy));
+    if (valid) {
+      if (l == 0) {
+        dgate[vid] = dg;
+        delta[((long)(tok / T) * H + h) * T + tok % T] = dl;
+      }
+      stv(dy + at, l, d);
     }
-    __nv_bfloat16* o = dy + wid * 128 + lane * 4;
-    st2(o, d.v[0], d.v[1]);
-    st2(o + 2, d.v[2], d.v[3]);
   }
   if (alpha != nullptr) {
     __syncthreads();
@@ -480,6 +547,13 @@ __global__ void gate_bwd_kernel(const float* __restrict__ dgate, const float* __
 
 inline int rc() { return cudaGetLastError() == cudaSuccess ? 0 : -5; }
 
+// The per-head vector kernels count vectors in 32 bits and use 16-byte accesses.
+inline bool vectors_ok(long n, std::initializer_list<const void*> ptrs) {
+  for (const void* p : ptrs)
+    if ((reinterpret_cast<uintptr_t>(p) & 15) != 0) return false;
+  return n <= 0x7fffffffL - kThreads;
+}
+
 constexpr int kIhaMaxHeads = 32;     // 2 x 32 registers of columns per thread
 constexpr int kIhaMaxDmixHeads = 20; // staging of iha_mix_bwd_mix_kernel in 48 KB of static shared memory
 
@@ -531,8 +605,9 @@ extern "C" int sr_qkv_prep_fwd(const void* qkv, const void* ve, const float* gat
                                cudaStream_t s) {
   const long n = tokens * H;
   if (n <= 0) return 0;
-  qkv_prep_fwd_kernel<<<(unsigned)((n + kWarpsPerBlock - 1) / kWarpsPerBlock), kThreads, 0, s>>>(
-      BF(qkv), BF(ve), gate, BF(cosb), BF(sinb), BFM(q), BFM(k), BFM(v), tokens, H, T, eps, key_offset);
+  if (!vectors_ok(n, {qkv, ve, cosb, sinb, q, k, v})) return -2;
+  qkv_prep_fwd_kernel<<<(unsigned)((n + kVecPerBlock - 1) / kVecPerBlock), kThreads, 0, s>>>(
+      BF(qkv), BF(ve), gate, BF(cosb), BF(sinb), BFM(q), BFM(k), BFM(v), n, H, T, eps, key_offset);
   return rc();
 }
 extern "C" int sr_qkv_prep_bwd(const void* qkv, const void* ve, const float* gate, const void* cosb, const void* sinb,
@@ -541,8 +616,9 @@ extern "C" int sr_qkv_prep_bwd(const void* qkv, const void* ve, const float* gat
                                cudaStream_t s) {
   const long n = tokens * H;
   if (n <= 0) return 0;
-  qkv_prep_bwd_kernel<<<(unsigned)((n + kWarpsPerBlock - 1) / kWarpsPerBlock), kThreads, 0, s>>>(
-      BF(qkv), BF(ve), gate, BF(cosb), BF(sinb), BF(dq), BF(dk), BF(dv), BFM(dqkv), BFM(dve), dgate, tokens, H, T, eps,
+  if (!vectors_ok(n, {qkv, ve, cosb, sinb, dq, dk, dv, dqkv, dve, dv_extra})) return -2;
+  qkv_prep_bwd_kernel<<<(unsigned)((n + kVecPerBlock - 1) / kVecPerBlock), kThreads, 0, s>>>(
+      BF(qkv), BF(ve), gate, BF(cosb), BF(sinb), BF(dq), BF(dk), BF(dv), BFM(dqkv), BFM(dve), dgate, n, H, T, eps,
       nullptr, key_offset, BF(dv_extra));
   return rc();
 }
@@ -553,8 +629,9 @@ extern "C" int sr_qkv_prep_bwd_f32dq(const void* qkv, const void* ve, const floa
                                      const void* dv_extra, cudaStream_t s) {
   const long n = tokens * H;
   if (n <= 0) return 0;
-  qkv_prep_bwd_kernel<<<(unsigned)((n + kWarpsPerBlock - 1) / kWarpsPerBlock), kThreads, 0, s>>>(
-      BF(qkv), BF(ve), gate, BF(cosb), BF(sinb), nullptr, BF(dk), BF(dv), BFM(dqkv), BFM(dve), dgate, tokens, H, T, eps,
+  if (!vectors_ok(n, {qkv, ve, cosb, sinb, dq_f32, dk, dv, dqkv, dve, dv_extra})) return -2;
+  qkv_prep_bwd_kernel<<<(unsigned)((n + kVecPerBlock - 1) / kVecPerBlock), kThreads, 0, s>>>(
+      BF(qkv), BF(ve), gate, BF(cosb), BF(sinb), nullptr, BF(dk), BF(dv), BFM(dqkv), BFM(dve), dgate, n, H, T, eps,
       dq_f32, key_offset, BF(dv_extra));
   return rc();
 }
@@ -564,8 +641,8 @@ extern "C" int sr_attn_post_fwd(const void* y, const void* v, const float* gate,
                                 int H, float xsa_eps, cudaStream_t s) {
   const long n = tokens * H;
   if (n <= 0) return 0;
-  if (H > 64) return -2;
-  long blocks = (n + kWarpsPerBlock - 1) / kWarpsPerBlock;
+  if (H > 64 || !vectors_ok(n, {y, alpha != nullptr ? v : nullptr, out})) return -2;
+  long blocks = (n + kVecPerBlock - 1) / kVecPerBlock;
   const long cap = (long)sm_count() * 16;
   if (blocks > cap) blocks = cap;
   attn_post_fwd_kernel<<<(unsigned)blocks, kThreads, 0, s>>>(BF(y), BF(v), gate, alpha, BFM(out), n, H, xsa_eps);
@@ -579,7 +656,8 @@ extern "C" int sr_attn_post_bwd(const void* g, const void* y, const void* v, con
   const long n = tokens * H;
   if (n <= 0) return 0;
   if (H > 64 || (alpha != nullptr && (dv_x == nullptr || dalpha == nullptr))) return -2;
-  long blocks = (n + kWarpsPerBlock - 1) / kWarpsPerBlock;
+  if (!vectors_ok(n, {g, y, alpha != nullptr ? v : nullptr, dy, alpha != nullptr ? dv_x : nullptr})) return -2;
+  long blocks = (n + kVecPerBlock - 1) / kVecPerBlock;
   const long cap = (long)sm_count() * 8;
   if (blocks > cap) blocks = cap;
   attn_post_bwd_kernel<<<(unsigned)blocks, kThreads, 0, s>>>(BF(g), BF(y), BF(v), gate, alpha, BFM(dy), dgate, delta,
