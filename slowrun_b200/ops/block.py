@@ -10,12 +10,15 @@ stochastic depth as a blend with the block input.
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 from torch.autograd import Function
 
 from . import _lib
 from . import functional as ops
 from .attention import current_impl
+from .flash_attention import DEFAULT_BKV, NativeAttention
 from .gemm import gemm
 
 P, I, L, F32, ULL = _lib.c_void_p, _lib.c_int, _lib.ctypes.c_long, _lib.c_float, _lib.ctypes.c_ulonglong
@@ -28,7 +31,7 @@ def _call(name, argtypes, *args):
 
 
 def _sp():
-    return torch.cuda.current_stream().cuda_stream
+    return _lib.stream_ptr()
 
 
 def _rmsnorm_fwd(x, eps):
@@ -139,6 +142,142 @@ def _gate_bwd(dgate, gate, a, w_param, da, H, nc, scale):
           scale, _sp())
 
 
+# ------------------------------------------------------------------ the launches in one host call (csrc/block_launch.cu)
+# Field by field the structs of that file.
+class _Shape(ctypes.Structure):
+    _fields_ = [("M", ctypes.c_longlong)] + \
+        [(n, I) for n in "B T C H hdim window key_offset do_mix attn_bkv gate_nc ve_gate_nc".split()] + \
+        [(n, F32) for n in "eps xsa_eps scale p_attn p_mlp".split()] + [("seed1", ULL), ("seed2", ULL)] + \
+        [(n, P) for n in "drop_state status rl xl sw ve_w mixes qkv_w gate_w ve_gate_w cosb sinb xsa proj_w gf_w mo_w".split()]
+
+
+class _FwdArgs(ctypes.Structure):
+    _fields_ = [("s", _Shape)] + [(n, P) for n in (
+        "xp x0 sk x a ve w_mix qkv agate ve_gate q k v y lse y2 o x_mid n gf hdn mo keep out").split()]
+
+
+class _BwdArgs(ctypes.Structure):
+    _fields_ = [("s", _Shape)] + [(n, P) for n in (
+        "g xp x0 sk x a ve w_qkv qkv agate ve_gate q k v y lse y2 x_mid n gf hdn keep "
+        "dmo g_mid g_in dhdn dgf dn g_mid_tot d_o dy2 dy dagate delta dv_x dq dk dv dqkv dve dvegate da dwp "
+        "dxp dx0 dsk g_mo g_gf g_proj g_qkv g_mix g_gate g_ve_gate g_ve g_rl g_xl g_sw g_xsa").split()]
+
+
+def _block_call(name, args):
+    n = _lib.fn(name, [P, P])(ctypes.addressof(args), _sp())
+    if n < 0:
+        raise RuntimeError(f"{name}: launcher {-n // 1000} of the block returned -{-n % 1000}")
+    _lib.launch_count += n - 1
+
+
+def _one_call(model, block, ve_lin, impl, C) -> bool:
+    """Whether the block runs through csrc/block_launch.cu: the in-tree attention, heads of 128 that make up the whole width,
+    dense bf16 weights, and (with IHA) the three mixing matrices next to each other and a head count the kernels know. What
+    is left goes launcher by launcher below."""
+    attn, mlp = block.attn, block.mlp
+    if not (type(impl) is NativeAttention and impl.has_bwd and attn.n_head * 128 == C and mlp is not None):
+        return False
+    ws = [attn.fused["qkv_w16"], attn.fused["proj_w16"], mlp.fused["gf_w16"], mlp.fused["proj_w16"]]
+    if ve_lin is not None:
+        ws.append(ve_lin.fused["w16"])
+    if any(w is None or not w.is_contiguous() for w in ws):
+        return False
+    if attn.use_iha:
+        return attn.n_head <= 32 and _stacked_mixes(model, attn, attn.n_head, ws[0].device)[1] is not None
+    return True
+
+
+def _shape(model, block, i, j, do_mix, ve_lin, mixes, xsa, dims, hdim, koff, window, scale, p_attn, p_mlp, seed1, seed2, eps, device):
+    B, T, C, H, D = dims
+    attn, mlp = block.attn, block.mlp
+    w = -1 if (window is None or window < 0 or window >= T) else int(window)
+    pt = _lib.ptr
+    return _Shape(
+        B * T, B, T, C, H, hdim, w, koff, int(do_mix), DEFAULT_BKV, attn.attn_gate_channels,
+        attn.ve_gate_channels if ve_lin is not None else 0, eps, float(attn.xsa_eps),
+        float(scale) if scale is not None else D ** -0.5, p_attn, p_mlp, seed1, seed2, ops.dropout_state(device).data_ptr(),
+        _lib.status_buffer(device).data_ptr(),
+        model.resid_lambdas.data_ptr() + 4 * i if do_mix else 0, model.x0_lambdas.data_ptr() + 4 * i if do_mix else 0,
+        model.skip_weights.data_ptr() + 4 * j if do_mix else 0, ve_lin.fused["w16"].data_ptr() if ve_lin is not None else 0,
+        pt(mixes), attn.fused["qkv_w16"].data_ptr(), attn.attn_gate.weight.data_ptr(),
+        attn.ve_gate.weight.data_ptr() if ve_lin is not None else 0, model.rotary.cos.data_ptr(), model.rotary.sin.data_ptr(),
+        xsa.data_ptr() + 4 * i * H if xsa is not None else 0, attn.fused["proj_w16"].data_ptr(), mlp.fused["gf_w16"].data_ptr(),
+        mlp.fused["proj_w16"].data_ptr())
+
+
+def _forward_one_call(model, block, i, j, do_mix, ve_lin, window, scale, training, xp, x0, sk, dims, eps):
+    """The forward of _BlockFn through one host call; returns (out, what the backward needs)."""
+    B, T, C, H, D = dims
+    M = B * T
+    attn, mlp = block.attn, block.mlp
+    dev = xp.device
+    bf16 = lambda *s: torch.empty(s, dtype=torch.bfloat16, device=dev)      # noqa: E731
+    fp32 = lambda *s: torch.empty(s, dtype=torch.float32, device=dev)       # noqa: E731
+    hdim = mlp.fused["gf_w16"].size(0) // 2
+    x, a = (bf16(M, C) if do_mix else xp), bf16(M, C)
+    ve, ve_gate = (bf16(M, C), fp32(M, H)) if ve_lin is not None else (None, None)
+    mixes, w_qkv = None, attn.fused["qkv_w16"]
+    if attn.use_iha:
+        mixes, _ = _stacked_mixes(model, attn, H, dev)
+        w_qkv = torch.empty_like(w_qkv)
+    qkv, agate = bf16(M, 3 * C), fp32(M, H)
+    q, k, v, y, y2 = (bf16(B, T, H, D) for _ in range(5))
+    lse = fp32(B, H, T)
+    o, x_mid, n, mo, out = (bf16(M, C) for _ in range(5))
+    gf, hdn = bf16(M, 2 * hdim), bf16(M, hdim)
+    koff = int(bool(attn.use_key_offset) and T > 1)
+    xsa = model.xsa_alphas if (do_mix and model._xsa_enabled(i)) else None
+    p_attn = float(attn.dropout) if training else 0.0
+    p_mlp = float(mlp.dropout) if training else 0.0
+    seed1 = ops.next_dropout_seed() if p_attn > 0 else 0
+    seed2 = ops.next_dropout_seed() if p_mlp > 0 else 0
+    keep = (torch.rand((), device=dev) >= block.drop_prob).float() if training and block.drop_prob > 0 else None
+    s = _shape(model, block, i, j, do_mix, ve_lin, mixes, xsa, dims, hdim, koff, window, scale, p_attn, p_mlp, seed1, seed2, eps, dev)
+    _block_call("sr_block_fwd", _FwdArgs(s, *map(_lib.ptr, (
+        xp, x0, sk, x, a, ve, w_qkv if mixes is not None else None, qkv, agate, ve_gate, q, k, v, y, lse, y2, o, x_mid, n, gf, hdn, mo,
+        keep, out))))
+    saved = (x, a, ve, mixes, w_qkv, qkv, agate, ve_gate, (q, k, v, y, lse, s.scale, s.window), y, y2, x_mid, n, gf, hdn, keep, v, xsa,
+             koff)
+    return out, saved, (p_attn, p_mlp, seed1, seed2)
+
+
+def _backward_one_call(saved, meta, g, xp, x0, sk, window, scale):
+    """The backward of _BlockFn through one host call: weight gradients are accumulated, returns (dxp, dx0, dsk)."""
+    x, a, ve, mixes, w_qkv, qkv, agate, ve_gate, (q, k, v, _, lse, _, _), y, y2, x_mid, n, gf, hdn, keep, _, xsa, koff = saved
+    model, block, i, j, do_mix, ve_lin, p_attn, p_mlp, seed1, seed2, eps, _, dims, has_x0, has_skip = meta
+    B, T, C, H, D = dims
+    M = B * T
+    attn, mlp = block.attn, block.mlp
+    fz, mz = attn.fused, mlp.fused
+    dev = g.device
+    bf16 = lambda *s: torch.empty(s, dtype=torch.bfloat16, device=dev)      # noqa: E731
+    fp32 = lambda *s: torch.empty(s, dtype=torch.float32, device=dev)       # noqa: E731
+    hdim = gf.size(1) // 2
+    dmo, dn, g_mid_tot, d_o, dy2, da, dxp = (bf16(M, C) for _ in range(7))
+    g_mid, g_in = (bf16(M, C), bf16(M, C)) if keep is not None else (None, None)
+    dhdn, dgf, dqkv = bf16(M, hdim), bf16(M, 2 * hdim), bf16(M, 3 * C)
+    dy, dk, dv = (bf16(B, T, H, D) for _ in range(3))
+    dv_x = bf16(B, T, H, D) if xsa is not None else None
+    dagate, delta, dq = fp32(M, H), fp32(B, H, T), fp32(B, T, H, D)
+    dve, dvegate = (bf16(M, C), fp32(M, H)) if ve is not None else (None, None)
+    dwp = torch.empty_like(w_qkv) if mixes is not None else None
+    dmix = _stacked_mixes(model, attn, H, dev)[1] if mixes is not None else None
+    dx0 = bf16(M, C) if (do_mix or ve is not None) else None
+    dsk = bf16(M, C) if has_skip and do_mix else None
+    s = _shape(model, block, i, j, do_mix, ve_lin, mixes, xsa, dims, hdim, koff, window, scale, p_attn, p_mlp, seed1, seed2, eps, dev)
+    pt = _lib.ptr
+    scalars = (model.resid_lambdas.grad.data_ptr() + 4 * i, model.x0_lambdas.grad.data_ptr() + 4 * i,
+               model.skip_weights.grad.data_ptr() + 4 * j if sk is not None else 0) if do_mix else (0, 0, 0)
+    _block_call("sr_block_bwd", _BwdArgs(
+        s, *map(pt, (g, xp, x0, sk, x, a, ve, w_qkv, qkv, agate, ve_gate, q, k, v, y, lse, y2, x_mid, n, gf, hdn, keep,
+                     dmo, g_mid, g_in, dhdn, dgf, dn, g_mid_tot, d_o, dy2, dy, dagate, delta, dv_x, dq, dk, dv, dqkv, dve, dvegate,
+                     da, dwp, dxp, dx0, dsk, mz["proj_grad"], mz["gf_grad"], fz["proj_grad"], fz["qkv_grad"], dmix,
+                     attn.attn_gate.weight.grad, attn.ve_gate.weight.grad if ve is not None else None,
+                     ve_lin.fused["grad"] if ve is not None else None)), *scalars,
+        xsa.grad.data_ptr() + 4 * i * H if xsa is not None else 0))
+    return dxp, dx0, dsk
+
+
 class _BlockFn(Function):
     @staticmethod
     def forward(ctx, x_prev, x0, skip, model, block, i, j, do_mix, ve_lin, window, scale, training):
@@ -158,6 +297,15 @@ class _BlockFn(Function):
         if skip is not None:
             sk = skip.reshape(M, C)
             sk = sk if sk.is_contiguous() else sk.contiguous()
+        if _one_call(model, block, ve_lin, impl, C):
+            out, saved, (p_attn, p_mlp, seed1, seed2) = _forward_one_call(
+                model, block, i, j, do_mix, ve_lin, window, scale, training, xp, x0_2, sk, (B, T, C, H, D), eps)
+            ctx.save_for_backward(xp, x0_2 if x0_2 is not None else xp.new_empty(0), sk if sk is not None else xp.new_empty(0))
+            ctx.t = saved
+            ctx.meta = (model, block, i, j, do_mix, ve_lin, p_attn, p_mlp, seed1, seed2, eps, impl, (B, T, C, H, D),
+                        x0 is not None, skip is not None)
+            ctx.attn_args = (window, scale)
+            return out.view(B, T, C)
         # ---- lambda mix
         if do_mix:
             x, a = torch.empty_like(xp), torch.empty_like(xp)
@@ -219,6 +367,7 @@ class _BlockFn(Function):
         ctx.t = (x, a, ve, mixes, w_qkv, qkv, agate, ve_gate, attn_saved, y, y2, x_mid, n, gf, hdn, keep, v, xsa, koff)
         ctx.meta = (model, block, i, j, do_mix, ve_lin, p_attn, p_mlp, seed1, seed2, eps, impl, (B, T, C, H, D),
                     x0 is not None, skip is not None)
+        ctx.attn_args = (window, scale)
         return out.view(B, T, C)
 
     @staticmethod
@@ -233,6 +382,11 @@ class _BlockFn(Function):
         fz, mz = attn.fused, mlp.fused
         g = g_out.reshape(M, C)
         g = g if g.is_contiguous() else g.contiguous()
+        if _one_call(model, block, ve_lin, impl, C) and (do_mix or keep is None):
+            saved = (x, a, ve, mixes, w_qkv, qkv, agate, ve_gate, attn_saved, y, y2, x_mid, n, gf, hdn, keep, v, xsa, koff)
+            dxp, dx0, dsk = _backward_one_call(saved, ctx.meta, g, xp, x0_2 if has_x0 else None, sk if has_skip else None,
+                                               *ctx.attn_args)
+            return tuple(t.view(B, T, C) if t is not None else None for t in (dxp, dx0, dsk)) + (None,) * 9
         # ---- MLP branch
         dmo, g_mid, g_in = _dropout_add_bwd(g, p_mlp, seed2, keep)
         if keep is None:

@@ -33,6 +33,16 @@ def _as3d(t: torch.Tensor):
     raise ValueError(f"expected a 2-D or 3-D tensor, got {tuple(t.shape)}")
 
 
+def _dims3d(t: torch.Tensor):
+    """Shape and strides of a 2-D or 3-D tensor as (batch, rows, cols); a 2-D one gets the strides `unsqueeze(0)` gives it."""
+    shape, stride = tuple(t.shape), t.stride()
+    if len(shape) == 2:
+        return (1,) + shape, (shape[0] * stride[0],) + stride
+    if len(shape) == 3:
+        return shape, stride
+    raise ValueError(f"expected a 2-D or 3-D tensor, got {shape}")
+
+
 def _check_operand(t: torch.Tensor, name: str):
     if t.dtype != torch.bfloat16:
         raise TypeError(f"{name} must be bfloat16, got {t.dtype}")
@@ -71,40 +81,30 @@ def gemm(a, b, out=None, cin=None, *, a_mn=False, b_mn=False, alpha=1.0, beta=0.
         raise TypeError("row_scale must be a contiguous float32 CUDA tensor")
     _check_operand(a, "a")
     _check_operand(b, "b")
-    A, B = _as3d(a), _as3d(b)
-    batch = A.shape[0]
-    if a_mn:
-        K, M = A.shape[1], A.shape[2]
-    else:
-        M, K = A.shape[1], A.shape[2]
-    if b_mn:
-        Kb, N = B.shape[1], B.shape[2]
-    else:
-        N, Kb = B.shape[1], B.shape[2]
-    if Kb != K or B.shape[0] != batch:
+    (batch, a1, a2), (sa, lda, _) = _dims3d(a)
+    (bb, b1, b2), (sb, ldb, _) = _dims3d(b)
+    M, K = (a2, a1) if a_mn else (a1, a2)
+    N, Kb = (b2, b1) if b_mn else (b1, b2)
+    if Kb != K or bb != batch:
         raise ValueError(f"shape mismatch: A {tuple(a.shape)} (a_mn={a_mn}) vs B {tuple(b.shape)} (b_mn={b_mn})")
     if out is None:
-        out = torch.empty((batch, M, N), dtype=out_dtype, device=a.device)
-        if a.dim() == 2:
-            out = out[0]
-    O = _as3d(out)
-    if O.shape != (batch, M, N) or O.stride(-1) != 1:
+        out = torch.empty((M, N) if a.dim() == 2 else (batch, M, N), dtype=out_dtype, device=a.device)
+    oshape, (so, ldo, o_inner) = _dims3d(out)
+    if oshape != (batch, M, N) or o_inner != 1:
         raise ValueError(f"bad output shape/stride {tuple(out.shape)}")
-    if O.dtype not in (torch.bfloat16, torch.float32):
+    if out.dtype not in (torch.bfloat16, torch.float32):
         raise TypeError("output must be bfloat16 or float32")
-    CI = None
+    sc = ldc = 0
+    cin_fp32 = False
     if cin is not None:
-        CI = _as3d(cin)
-        if CI.shape != (batch, M, N) or CI.stride(-1) != 1 or CI.dtype not in (torch.bfloat16, torch.float32):
+        cshape, (sc, ldc, c_inner) = _dims3d(cin)
+        if cshape != (batch, M, N) or c_inner != 1 or cin.dtype not in (torch.bfloat16, torch.float32):
             raise ValueError("bad cin")
+        cin_fp32 = cin.dtype == torch.float32
     f = _lib.fn("sr_gemm_bf16", _ARGTYPES)
-    rc = f(A.data_ptr(), B.data_ptr(), O.data_ptr(), _lib.ptr(CI), M, N, K, batch,
-           A.stride(1), B.stride(1), O.stride(1), CI.stride(1) if CI is not None else 0,
-           A.stride(0), B.stride(0), O.stride(0), CI.stride(0) if CI is not None else 0,
-           int(a_mn), int(b_mn), int(O.dtype == torch.float32),
-           int(CI is not None and CI.dtype == torch.float32),
-           float(alpha), float(beta), _lib.ptr(alpha_t), _lib.ptr(row_scale), int(sym), int(bn), int(max_ctas),
-           _lib.status_buffer(a.device).data_ptr(), _lib.stream_ptr())
+    rc = f(a.data_ptr(), b.data_ptr(), out.data_ptr(), _lib.ptr(cin), M, N, K, batch, lda, ldb, ldo, ldc, sa, sb, so, sc,
+           int(a_mn), int(b_mn), int(out.dtype == torch.float32), int(cin_fp32), float(alpha), float(beta), _lib.ptr(alpha_t),
+           _lib.ptr(row_scale), int(sym), int(bn), int(max_ctas), _lib.status_buffer(a.device).data_ptr(), _lib.stream_ptr())
     _lib.check_rc(rc, "sr_gemm_bf16")
     return out
 
