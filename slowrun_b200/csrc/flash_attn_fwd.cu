@@ -22,7 +22,7 @@ constexpr int kThreads = 192;
 constexpr uint32_t kQBytes = BQ * D * 2;           // 32 KB
 constexpr uint32_t kQHalf = BQ * 128;              // one 64-column half of a 128-row tile: 128 rows x 128 B
 
-// BKV = keys per tile; with 64, two CTAs fit an SM and their softmax and MMA phases overlap.
+// BKV = keys per tile. 128: one CTA per SM; 64: two CTAs per SM (their softmax and MMA phases overlap).
 template <int BKV>
 struct FwdCfg {
   static constexpr uint32_t kKVBytes = BKV * D * 2;       // K or V tile
@@ -685,31 +685,12 @@ int launch_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& 
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
-// Which of the two kernels: the pair kernel has half as many, twice as long blocks, and a block starts and ends with one of
-// its two tiles alone. It needs blocks for (nearly) every SM and rows that see a few key tiles. us, 64-key kernel / pair:
-//   blocks 32, (1, 2048, 4) window 1024: 22.5 / 25.9      blocks 64, (1, 2048, 8)-like (1, 777, 8): 16.1 / 17.9
-//   blocks 128, (4, 2048, 4) window 1024: 29.3 / 26.4     blocks 256, (8, 1024, 8) window 512 (384 visible keys): 35.2 / 36.5
-//   (32, 2048, 8) window 512 (449 visible keys): 240 / 239, full causal: 404 / 348; (4, 2048, 14) window 1792: 113 / 98
-static bool use_pair_kernel(int B, int T, int H, int window) {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  }
-  const long blocks = (long)((T + 255) / 256) * B * H;
-  const double w = window < 0 ? T : (window + 1 < T ? window + 1 : T);
-  return blocks * 5 >= sms * 4 && w - w * (w - 1) / (2.0 * T) >= 448;
-}
-
 // q, k, v: (B, T, H, 128) bf16 with token stride ld_* elements (contiguous tensors: H*128); out contiguous;
-// lse: fp32 (B, H, T), natural log of sum exp(scale * s). window < 0 = full causal. bkv: 64 = one query tile per block and
-// 64-key tiles, 128 = the pair kernel, 0 = choose.
+// lse: fp32 (B, H, T), natural log of sum exp(scale * s). window < 0 = full causal. bkv: 64 or 128 keys per tile.
 extern "C" int sr_flash_attn_fwd(const void* q, const void* k, const void* v, void* out, float* lse, int B, int T, int H,
                                  long ld_q, long ld_k, long ld_v, int window, float scale, int bkv, int* status,
                                  cudaStream_t stream) {
   if (B <= 0 || T <= 0 || H <= 0) return 0;
-  if (bkv == 0) bkv = use_pair_kernel(B, T, H, window) ? 128 : 64;
   if (bkv != 64 && bkv != 128) return -2;
   CUtensorMap mq, mk, mv;
   int rc;

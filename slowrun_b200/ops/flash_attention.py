@@ -28,7 +28,7 @@ def native_available() -> bool:
     return _has("sr_flash_attn_fwd")
 
 
-DEFAULT_BKV = int(os.environ.get("SLOWRUN_ATTN_BKV", "0"))     # 0: chosen by the launcher from the sizes
+DEFAULT_BKV = int(os.environ.get("SLOWRUN_ATTN_BKV", "64"))
 
 
 def native_fwd(q, k, v, window, scale, bkv=None):
@@ -43,7 +43,7 @@ def native_fwd(q, k, v, window, scale, bkv=None):
     sc = float(scale) if scale is not None else D ** -0.5
     rc = _lib.fn("sr_flash_attn_fwd", [P] * 5 + [I, I, I, L, L, L, I, F32, I, P, P])(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(), B, T, H, q.stride(1), k.stride(1),
-        v.stride(1), w, sc, int(DEFAULT_BKV if bkv is None else bkv), _lib.status_buffer(q.device).data_ptr(), _lib.stream_ptr())
+        v.stride(1), w, sc, int(bkv or DEFAULT_BKV), _lib.status_buffer(q.device).data_ptr(), _lib.stream_ptr())
     _lib.check_rc(rc, "sr_flash_attn_fwd")
     return out, lse, sc, w
 
