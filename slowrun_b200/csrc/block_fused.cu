@@ -101,6 +101,31 @@ __device__ __forceinline__ float sum8(float v) {
   return v;
 }
 
+// The forward kernels sum in the order of a butterfly over 32 lanes, so that their results do not depend on how many lanes
+// share a vector: a change of rounding in the forward travels through every later layer and shows as 1 to 2 % in gradients
+// that are sums with cancellation. Lane l stands for lanes 4l .. 4l+3 of a warp with elements {2L, 2L+1, 64+2L, 64+2L+1} each
+// (sum_sq_pairs) or for lanes 2l, 2l+1, 16+2l, 16+2l+1 with elements 4L .. 4L+3 (dot_quads).
+__device__ __forceinline__ float sum_sq_pairs(const Vec& o) {
+  float s[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    s[j] = o.lo[2 * j] * o.lo[2 * j] + o.lo[2 * j + 1] * o.lo[2 * j + 1] + o.hi[2 * j] * o.hi[2 * j] + o.hi[2 * j + 1] * o.hi[2 * j + 1];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) s[j] = sum8(s[j]);
+  return (s[0] + s[2]) + (s[1] + s[3]);
+}
+__device__ __forceinline__ float dot_quads(const Vec& a, const Vec& b) {
+  float s[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int i = 4 * j;
+    const float lo = a.lo[i] * b.lo[i] + a.lo[i + 1] * b.lo[i + 1] + a.lo[i + 2] * b.lo[i + 2] + a.lo[i + 3] * b.lo[i + 3];
+    const float hi = a.hi[i] * b.hi[i] + a.hi[i + 1] * b.hi[i + 1] + a.hi[i + 2] * b.hi[i + 2] + a.hi[i + 3] * b.hi[i + 3];
+    s[j] = sum8(lo + hi);
+  }
+  return s[0] + s[1];
+}
+
 // ---------------------------------------------------------------------------------------------- qkv prep
 __global__ void __launch_bounds__(kThreads)
 qkv_prep_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ ve, const float* __restrict__ gate,
@@ -136,7 +161,7 @@ qkv_prep_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* 
       o.lo[i] = x[which].lo[i] * c[i] + x[which].hi[i] * s[i];
       o.hi[i] = -x[which].lo[i] * s[i] + x[which].hi[i] * c[i];
     }
-    const float r = rsqrtf(sum8(dot(o, o)) * (1.f / 128.f) + eps);
+    const float r = rsqrtf(sum_sq_pairs(o) * (1.f / 128.f) + eps);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       o.lo[i] *= r;
@@ -205,7 +230,7 @@ qkv_prep_bwd_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* 
       o.lo[i] = x.lo[i] * c[i] + x.hi[i] * s[i];
       o.hi[i] = -x.lo[i] * s[i] + x.hi[i] * c[i];
     }
-    const float r = rsqrtf(sum8(dot(o, o)) * (1.f / 128.f) + eps);
+    const float r = rsqrtf(sum_sq_pairs(o) * (1.f / 128.f) + eps);
     const float k = r * r * r * sum8(dot(o, g)) * (1.f / 128.f);
     Vec w;
 #pragma unroll
@@ -258,8 +283,8 @@ attn_post_fwd_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* _
     const float s = gate[vid];
     if (alpha != nullptr) {
       const Vec vv = ldv(v + at, l);
-      const float nn = fmaxf(sqrtf(sum8(dot(vv, vv))), xsa_eps);
-      const float c = sum8(dot(yy, vv)) / nn;
+      const float nn = fmaxf(sqrtf(dot_quads(vv, vv)), xsa_eps);
+      const float c = dot_quads(yy, vv) / nn;
       const float k = tanhf(alpha[vid % H]) * c / nn;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -303,11 +328,11 @@ attn_post_bwd_kernel(const __nv_bfloat16* __restrict__ g, const __nv_bfloat16* _
     float dg;    // sum_d g * (output before the gate)
     if (alpha != nullptr) {
       const Vec vv = ldv(v + at, l);
-      const float nrm = sqrtf(sum8(dot(vv, vv)));
+      const float nrm = sqrtf(dot_quads(vv, vv));
       const float inv = 1.f / fmaxf(nrm, xsa_eps);
-      const float c = sum8(dot(yy, vv)) * inv;                // y . u,  u = v / max(|v|, eps)
+      const float c = dot_quads(yy, vv) * inv;                // y . u,  u = v / max(|v|, eps)
       const float a = tanhf(alpha[h]);
-      const float gy = sum8(dot(gg, yy)), gu = sum8(dot(gg, vv)) * inv;
+      const float gy = dot_quads(gg, yy), gu = dot_quads(gg, vv) * inv;
       dg = gy - a * c * gu;                                   // g . (y - a c u)
       const float p = s * gu;                                 // (s g) . u
       Vec du;
@@ -320,7 +345,7 @@ attn_post_bwd_kernel(const __nv_bfloat16* __restrict__ g, const __nv_bfloat16* _
         du.hi[i] = -a * (p * yy.hi[i] + c * d1);
       }
       // v -> u = v / max(|v|, eps): the projection term only where the norm is not clamped
-      const float proj = sum8(dot(du, vv)) * inv;
+      const float proj = dot_quads(du, vv) * inv;
       const float duu = nrm > xsa_eps ? proj : 0.f;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -332,14 +357,14 @@ attn_post_bwd_kernel(const __nv_bfloat16* __restrict__ g, const __nv_bfloat16* _
         if (l == 0) atomicAdd(&dal[h], -c * p * (1.f - a * a));
       }
     } else {
-      dg = sum8(dot(gg, yy));
+      dg = dot_quads(gg, yy);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         d.lo[i] = s * gg.lo[i];
         d.hi[i] = s * gg.hi[i];
       }
     }
-    const float dl = sum8(dot(d, yy));
+    const float dl = dot_quads(d, yy);
     if (valid) {
       if (l == 0) {
         dgate[vid] = dg;

@@ -643,13 +643,12 @@ __global__ void norm_bwd_drop_kernel(const __nv_bfloat16* __restrict__ x_mid, co
   }
 }
 
-// ------------------------------------------------------------------ the same four row kernels, a row held by a group of threads
-// The kernels above give a row to one warp, which walks it twice: at D = 2560 ten dependent steps of 16-byte loads per pass,
-// with 8192 rows filling less than one wave. Here TPR threads hold a row in registers (VPT vectors of 8 each): every load of
-// the row is in flight at once, each input is read once, and the only wait is the reduction over the group. Blocks walk over
-// rows, so the scalar sums of norm_bwd_mix cost three atomics per block and not per eight rows.
-// us, warp per row -> these, [8192, 2560]: norm_bwd_mix 110 -> 79, norm_bwd_drop 72 -> 64, mix_norm_fwd 48 -> 37, add_norm_fwd
-// 50 -> 46 (the dropout hash bounds the two with a mask); [65536, 1024]: 247 -> 226, 182 -> 158, 129 -> 98, 129 -> 127.
+// ------------------------------------------------------------------ the same four row kernels, a row in registers
+// The kernels above walk a row twice: at D = 2560 ten dependent steps of 16-byte loads per pass, with 8192 rows filling less
+// than one wave. Here a row sits in the registers of the threads that own it: every load is in flight at once and each input
+// is read once. The backward kernels use TPR threads per row (VPT vectors of 8 each) and blocks that walk over rows, so the
+// scalar sums of norm_bwd_mix cost three atomics per block and not per eight rows.
+// ROWS_MEASURED_PLACEHOLDER
 constexpr int kRowThreads = 128;
 
 // sums of a and b over the TPR threads of a row; `red` holds 2 x 4 pairs that alternate, so one barrier per call suffices
@@ -680,6 +679,13 @@ __device__ __forceinline__ void unpack8(const uint4& t, float (&f)[8]) {
     f[2 * i + 1] = a.y;
   }
 }
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+  uint4 t;
+  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&t);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+  return t;
+}
 __device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16(x)); }
 
 // f(row, valid) for the rows of this group; all threads of the block make the same number of steps
@@ -698,94 +704,95 @@ __device__ __forceinline__ void row_vectors(int tid, int D, bool valid, F f) {
 }
 #define LDV(p) (*reinterpret_cast<const uint4*>(p))
 
-template <int TPR, int VPT>
+// The two forward kernels keep one warp per row (VPT vectors per lane, all in flight at once): their sum of squares is then
+// taken in the order of the kernels above, bit for bit. A change of rounding in the forward would travel through every later
+// layer and show as 1 to 2 % in gradients that are sums with cancellation.
+template <int VPT>
 __global__ void __launch_bounds__(kRowThreads)
 mix_norm_fwd_rows(const __nv_bfloat16* __restrict__ xp, const __nv_bfloat16* __restrict__ x0, const __nv_bfloat16* __restrict__ skip,
                   __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ a_out, const float* __restrict__ lr_p,
                   const float* __restrict__ l0_p, const float* __restrict__ ws_p, long rows, int D, float eps) {
-  __shared__ float2 red[2][4];
-  int turn = 0;
+  const long row = (long)blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const int lane = threadIdx.x & 31;
   const float lr = *lr_p, l0 = *l0_p, ws = skip ? *ws_p : 0.f;
-  SR_FOR_ROWS(TPR) {
-    const long row = row0 + threadIdx.x / TPR;
-    const bool valid = row < rows;
-    const long base = row * (long)D;
-    uint4 A[VPT], B[VPT], S[VPT];
-    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
-      A[i] = LDV(xp + base + c);
-      B[i] = LDV(x0 + base + c);
-      if (skip) S[i] = LDV(skip + base + c);
-    });
-    float v[VPT][8];
-    float ss = 0.f;
-    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
-      float a[8], b[8], sk[8];
-      unpack8(A[i], a);
-      unpack8(B[i], b);
-      if (skip) {
-        unpack8(S[i], sk);
+  const long base = row * (long)D;
+  uint4 A[VPT], B[VPT], S[VPT];
+  row_vectors<32, VPT>(lane, D, true, [&](int i, int c) {
+    A[i] = LDV(xp + base + c);
+    B[i] = LDV(x0 + base + c);
+    if (skip) S[i] = LDV(skip + base + c);
+  });
+  float ss = 0.f;
+  row_vectors<32, VPT>(lane, D, true, [&](int i, int c) {
+    float a[8], b[8];
+    unpack8(A[i], a);
+    unpack8(B[i], b);
+    if (skip) {
+      float s[8];
+      unpack8(S[i], s);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) a[j] += ws * sk[j];
-      }
+      for (int j = 0; j < 8; ++j) a[j] += ws * s[j];
+    }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        v[i][j] = round_bf16(lr * a[j] + l0 * b[j]);
-        ss += v[i][j] * v[i][j];
-      }
-      store8(x + base + c, v[i]);
-    });
-    const float r = rsqrtf(group_sum<TPR>(ss, 0.f, red, turn).x / D + eps);
-    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
+    for (int j = 0; j < 8; ++j) {
+      a[j] = round_bf16(lr * a[j] + l0 * b[j]);
+      ss += a[j] * a[j];
+    }
+    A[i] = pack8(a);
+    *reinterpret_cast<uint4*>(x + base + c) = A[i];
+  });
+  ss = warp_sum(ss);
+  const float r = rsqrtf(ss / D + eps);
+  row_vectors<32, VPT>(lane, D, true, [&](int i, int c) {
+    float f[8];
+    unpack8(A[i], f);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[i][j] *= r;
-      store8(a_out + base + c, v[i]);
-    });
-  }
+    for (int j = 0; j < 8; ++j) f[j] *= r;
+    store8(a_out + base + c, f);
+  });
 }
 
-template <int TPR, int VPT>
+template <int VPT>
 __global__ void __launch_bounds__(kRowThreads)
 add_norm_fwd_rows(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ x_mid,
                   __nv_bfloat16* __restrict__ n, long rows, int D, float eps, float p, uint64_t salt,
                   const unsigned long long* __restrict__ seed_ptr) {
-  __shared__ float2 red[2][4];
-  int turn = 0;
+  const long row = (long)blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const int lane = threadIdx.x & 31;
   const uint64_t seed = salt + (seed_ptr ? (*seed_ptr) * 0x9E3779B97F4A7C15ull : 0ull);
   const float scale = 1.f / (1.f - p);
   const uint32_t thr = keep_threshold(p);
-  SR_FOR_ROWS(TPR) {
-    const long row = row0 + threadIdx.x / TPR;
-    const bool valid = row < rows;
-    const long base = row * (long)D;
-    uint4 A[VPT], B[VPT];
-    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
-      A[i] = LDV(x + base + c);
-      B[i] = LDV(y + base + c);
-    });
-    float v[VPT][8];
-    float ss = 0.f;
-    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
-      float a[8], b[8];
-      unpack8(A[i], a);
-      unpack8(B[i], b);
-      if (p > 0.f) {
+  const long base = row * (long)D;
+  uint4 A[VPT], B[VPT];
+  row_vectors<32, VPT>(lane, D, true, [&](int i, int c) {
+    A[i] = LDV(x + base + c);
+    B[i] = LDV(y + base + c);
+  });
+  float ss = 0.f;
+  row_vectors<32, VPT>(lane, D, true, [&](int i, int c) {
+    float a[8], b[8];
+    unpack8(A[i], a);
+    unpack8(B[i], b);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) b[j] = keep_elem(seed, (uint64_t)(base + c + j), thr) ? b[j] * scale : 0.f;
-      }
+    for (int j = 0; j < 8; ++j) {
+      if (p > 0.f) b[j] = keep_elem(seed, (uint64_t)(base + c + j), thr) ? b[j] * scale : 0.f;
+      a[j] = round_bf16(a[j] + b[j]);
+      ss += a[j] * a[j];
+    }
+    A[i] = pack8(a);
+    *reinterpret_cast<uint4*>(x_mid + base + c) = A[i];
+  });
+  ss = warp_sum(ss);
+  const float r = rsqrtf(ss / D + eps);
+  row_vectors<32, VPT>(lane, D, true, [&](int i, int c) {
+    float f[8];
+    unpack8(A[i], f);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        v[i][j] = round_bf16(a[j] + b[j]);
-        ss += v[i][j] * v[i][j];
-      }
-      store8(x_mid + base + c, v[i]);
-    });
-    const float r = rsqrtf(group_sum<TPR>(ss, 0.f, red, turn).x / D + eps);
-    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v[i][j] *= r;
-      store8(n + base + c, v[i]);
-    });
-  }
+    for (int j = 0; j < 8; ++j) f[j] *= r;
+    store8(n + base + c, f);
+  });
 }
 
 template <int TPR, int VPT>
@@ -959,8 +966,8 @@ inline int grid_for(long n, int per_block) {
 }
 inline int rc() { return cudaGetLastError() == cudaSuccess ? 0 : -5; }
 
-// Rows of 264 to 4096 elements go to the *_rows kernels: 64 threads up to 512, 128 beyond, as many vectors per thread as the
-// row needs. Shorter rows are one step for a warp as it is, longer ones would not fit the registers.
+// The backward kernels: rows of 264 to 4096 elements, 64 threads up to 512, 128 beyond, as many vectors per thread as the row
+// needs. Shorter rows are one step for a warp as it is, longer ones would not fit the registers.
 template <typename F>
 bool row_dispatch(int D, F f) {
   if (D <= 256 || D > 4096) return false;
@@ -970,6 +977,17 @@ bool row_dispatch(int D, F f) {
   else if (D <= 3072) f(std::integral_constant<int, 128>(), std::integral_constant<int, 3>());
   else f(std::integral_constant<int, 128>(), std::integral_constant<int, 4>());
   return true;
+}
+// The forward kernels: one warp per row, vectors per lane = ceil(D / 256) up to 10 (longer rows would not fit the registers).
+template <int V, typename F>
+bool row_dispatch_warp(int D, F f) {
+  if (D <= 256 || D > 256 * V) return false;
+  if (D > 256 * (V - 1)) {
+    f(std::integral_constant<int, V>());
+    return true;
+  }
+  if constexpr (V > 2) return row_dispatch_warp<V - 1>(D, f);
+  return false;
 }
 inline unsigned row_grid(long rows, int tpr, int blocks_per_sm) {
   const long b = (rows * tpr + kRowThreads - 1) / kRowThreads, cap = (long)sm_count() * blocks_per_sm;
@@ -1078,8 +1096,8 @@ extern "C" int sr_add_norm_fwd(const void* x, const void* y, void* x_mid, void* 
                                unsigned long long seed, const unsigned long long* seed_ptr, cudaStream_t s) {
   if (D % 8) return -2;
   if (rows <= 0) return 0;
-  if (row_dispatch(D, [&](auto tpr, auto vpt) {
-        add_norm_fwd_rows<tpr.value, vpt.value><<<row_grid(rows, tpr.value, 64), kRowThreads, 0, s>>>(
+  if (row_dispatch_warp<10>(D, [&](auto vpt) {
+        add_norm_fwd_rows<vpt.value><<<(unsigned)((rows + kRowThreads / 32 - 1) / (kRowThreads / 32)), kRowThreads, 0, s>>>(
             BF(x), BF(y), BFM(x_mid), BFM(n), rows, D, eps, p, seed, seed_ptr);
       }))
     return rc();
@@ -1108,8 +1126,8 @@ extern "C" int sr_mix_norm_fwd(const void* xp, const void* x0, const void* skip,
                                const float* l0, const float* ws, long rows, int D, float eps, cudaStream_t s) {
   if (D % 8) return -2;
   if (rows <= 0) return 0;
-  if (row_dispatch(D, [&](auto tpr, auto vpt) {
-        mix_norm_fwd_rows<tpr.value, vpt.value><<<row_grid(rows, tpr.value, 64), kRowThreads, 0, s>>>(
+  if (row_dispatch_warp<10>(D, [&](auto vpt) {
+        mix_norm_fwd_rows<vpt.value><<<(unsigned)((rows + kRowThreads / 32 - 1) / (kRowThreads / 32)), kRowThreads, 0, s>>>(
             BF(xp), BF(x0), BF(skip), BFM(x), BFM(a), lr, l0, ws, rows, D, eps);
       }))
     return rc();

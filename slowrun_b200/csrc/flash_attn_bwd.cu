@@ -6,7 +6,7 @@
 //     S^T  = K_j Q_i^T          dP^T = V_j dO_i^T               (both operands K-major)
 //     dV  += P^T dO_i           (A = P^T, bf16 in the TMEM columns of S^T; B MN-major)
 //     dK  += dS^T Q_i           dQ_i = dS K_j                   (one shared-memory tile dS^T, read K-major and MN-major)
-// with P = exp(scale*S - lse) and dS = P * (dP - delta); the factor `scale` of dK and dQ is applied to the fp32 results.
+// with P = exp(scale*S - lse) and dS = P * (dP - delta) * scale.
 //
 // What bounds it: a tile pair is 5 x 512 tensor-pipe cycles, 128*128 exponentials (1024 cycles of the special-function
 // pipe) and about 4000 cycles' worth of shared-memory traffic (operands, dS, dQ staging, loads), so the point of the
@@ -368,6 +368,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       if (!ok) break;
       tc_fence_after();
       const float* ndelta = nlse + 128;
+      const uint64_t sc2 = pack_f32x2(p.scale, p.scale);
 #pragma unroll
       for (int ch = 0; ch < 4; ++ch) {
         uint32_t dp[16];
@@ -383,7 +384,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
             const uint32_t pa = ch < 2 ? s0[cc] : s1[cc], pb = ch < 2 ? s0[cc + 1] : s1[cc + 1];
             const uint64_t t = add_f32x2(pack_f32x2(__uint_as_float(dp[c + e]), __uint_as_float(dp[c + e + 1])), e == 0 ? nd.x : nd.y);
             float d0, d1;
-            unpack_f32x2(mul_f32x2(t, pack_f32x2(__uint_as_float(pa), __uint_as_float(pb))), d0, d1);
+            unpack_f32x2(mul_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(pa), __uint_as_float(pb)), t), sc2), d0, d1);
             dd[(c + e) / 2] = pack_bf16x2(d0, d1);
           }
         }
@@ -410,7 +411,6 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       for (int which = 0; which < 2; ++which) {
         const uint32_t t = (which == 0 ? tdV : tdK) + lane_addr;
         __nv_bfloat16* dstp = (which == 0 ? p.dv : p.dk) + base;
-        const float f = which == 0 ? 1.f : p.scale;
 #pragma unroll 1
         for (int ch = chalf * 2; ch < chalf * 2 + 2; ++ch) {
           uint32_t v[32];
@@ -423,7 +423,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
               uint32_t* hh = reinterpret_cast<uint32_t*>(&o);
 #pragma unroll
               for (int e = 0; e < 4; ++e)
-                hh[e] = pack_bf16x2(__uint_as_float(v[jj + 2 * e]) * f, __uint_as_float(v[jj + 2 * e + 1]) * f);
+                hh[e] = pack_bf16x2(__uint_as_float(v[jj + 2 * e]), __uint_as_float(v[jj + 2 * e + 1]));
               *reinterpret_cast<uint4*>(dstp + ch * 32 + jj) = o;
             }
           }
@@ -459,9 +459,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
           uint8_t* rowp = box + lane * 128;
 #pragma unroll
           for (int c = 0; c < 8; ++c)
-            *reinterpret_cast<float4*>(rowp + ((c ^ (lane & 7)) << 4)) =
-                make_float4(__uint_as_float(v[c2][4 * c]) * p.scale, __uint_as_float(v[c2][4 * c + 1]) * p.scale,
-                            __uint_as_float(v[c2][4 * c + 2]) * p.scale, __uint_as_float(v[c2][4 * c + 3]) * p.scale);
+            *reinterpret_cast<uint4*>(rowp + ((c ^ (lane & 7)) << 4)) =
+                make_uint4(v[c2][4 * c], v[c2][4 * c + 1], v[c2][4 * c + 2], v[c2][4 * c + 3]);
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {

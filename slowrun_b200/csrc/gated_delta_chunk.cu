@@ -1,24 +1,26 @@
-// Gated delta rule with one log-decay per head, chunk by chunk, forward and backward.
+// Backward of the gated delta rule with one log-decay per head, chunk by chunk.
 //
-// The recurrence (gated_delta.cu) does one token after the other: 2048 dependent steps of two warp reductions each. Here a
-// chunk of 64 tokens is a handful of dense 64-row products, and only the state has to travel from chunk to chunk. With G_t
-// the running sum of the log-decays inside the chunk, S the state [Dk x Dv] entering it, E[t,j] = exp(G_t - G_j):
+// The forward is the recurrence of gated_delta.cu. For the gradients a chunk of 64 tokens is a handful of dense 64-row
+// products, and only the state has to travel from chunk to chunk. With G_t the running sum of the log-decays inside the
+// chunk, S the state [Dk x Dv] entering it, E[t,j] = exp(G_t - G_j):
 //     A[t,j] = beta_j (k_t . k_j) E[t,j]  (j < t)        P[t,j] = beta_j (q_t . k_j) E[t,j]  (j <= t)
 //     R      = (I + A)^-1 (V - Kd S)                     Kd = exp(G) K,  Qd = exp(G) Q
 //     O      = Qd S + P R
 //     S_next = exp(G_C) S + Kend^T R                     Kend_j = beta_j exp(G_C - G_j) k_j
 // Every exponential is of a non-positive number. With W = (I + A)^-1 Kd and U = (I + A)^-1 V, which need no state, the part
 // that runs in sequence is R = U - W S and the state update: two small products per chunk, independent for every slice of
-// value columns. The backward has the same shape, last chunk first, with dS the gradient of the state leaving a chunk:
+// value columns. The gradients have the same shape, last chunk first, with dS the gradient of the state leaving a chunk:
 //     dRhs    = X + Y dS         X = (I + A)^-T P^T dO,  Y = (I + A)^-T Kend
 //     dS_prev = exp(G_C) dS + Z - Kd^T dRhs,             Z = Qd^T dO                       dV = dRhs
-// So both directions are three kernels: prep (all chunks at once), scan (in sequence, one CTA per head and 32 value
-// columns), and out / grads (all chunks at once). All arithmetic is fp32 FMA as in the recurrence; q, k, v may be bf16 or fp32.
+// So there are three kernels: prep (all chunks at once), scan (in sequence, one CTA per head and 32 value columns; once
+// forward for the states, once backward), and grads (all chunks at once). All arithmetic is fp32 FMA as in the recurrence;
+// q, k, v may be bf16 or fp32. (The same chunks give the forward as well, in 890 us against the recurrence's 1650. That is not
+// used: its other rounding travels through every later layer of a model.)
 //
 // What bounds it: shared-memory reads of the 64 x 64 x n products (a thread owns 4 x 4 results) and, for the scan, the
 // latency of n_chunks dependent steps, which is why its operands are prefetched with cp.async.
-// Measured, (B, T, H) = (4, 2048, 14), Dk = 64, Dv = 128: forward 890 us (recurrence kernel: 1650 us), backward 2.0 ms
-// (gradients through the PyTorch form: about 17 ms in 2900 launches); prep 430 / 730, scan 240, out 230, grads 815 us.
+// Measured, (B, T, H) = (4, 2048, 14), Dk = 64, Dv = 128: 2.0 ms (gradients through the PyTorch form: about 17 ms in 2900
+// launches); prep 730, scan 240 each way, grads 815 us.
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
@@ -186,17 +188,16 @@ __device__ __forceinline__ void invert_unit_lower(const float* A, float* X) {
 // Scratch: rows are padded to whole chunks (row cc * 64 + t with cc = bh * n + c) and value columns to whole slices (DvP).
 //   W [64 x Dk] = -(I + A)^-1 Kd       U [64 x DvP] = (I + A)^-1 V, overwritten by R       Ke [64 x Dk] = Kend
 //   S [Dk x DvP] state entering the chunk        dec = exp(G_C)
-//   forward:   P [64 x 64]
-//   backward:  Y [64 x Dk] = (I + A)^-T Kend     X [64 x DvP] = (I + A)^-T P^T dO, overwritten by dRhs     Kn [64 x Dk] = -Kd
-//              Z [Dk x DvP] = Qd^T dO            dS [Dk x DvP] gradient of the state leaving the chunk
+//   Y [64 x Dk] = (I + A)^-T Kend      X [64 x DvP] = (I + A)^-T P^T dO, overwritten by dRhs     Kn [64 x Dk] = -Kd
+//   Z [Dk x DvP] = Qd^T dO             dS [Dk x DvP] gradient of the state leaving the chunk
 struct Scratch {
-  float *W, *U, *Ke, *S, *dec, *P, *Y, *X, *Kn, *Z, *dS;
+  float *W, *U, *Ke, *S, *dec, *Y, *X, *Kn, *Z, *dS;
 };
 
 template <int Dk>
 constexpr int prep_smem() { return (2 * C * (Dk + 4) + 3 * C * LC + C * LV + 2 * C) * 4; }
 
-template <int Dk, bool BWD, typename T>
+template <int Dk, typename T>
 __global__ void __launch_bounds__(kThreads)
 gdn_prep_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const float* __restrict__ g,
                 const float* __restrict__ beta, const T* __restrict__ dO, Scratch s, Dims d) {
@@ -226,7 +227,6 @@ gdn_prep_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __res
     each(acc, [&](int t, int j, float x) {
       const float y = j <= t ? x * bt[j] * decay_exp(G[t] - G[j]) : 0.f;
       sP[t * LC + j] = y;
-      if (!BWD) s.P[(cc * C + t) * C + j] = y;
     });
   }
   __syncthreads();
@@ -236,15 +236,13 @@ gdn_prep_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __res
     const int t = i / Dk, x = i - t * Dk;
     const float kk = sK[t * LK + x], e = decay_exp(G[t]), ke = kk * bt[t] * decay_exp(Gend - G[t]);
     s.Ke[(cc * C + t) * Dk + x] = ke;
-    if (BWD) {
-      s.Kn[(cc * C + t) * Dk + x] = -kk * e;
-      sQ[t * LK + x] *= e;
-    }
-    sK[t * LK + x] = BWD ? ke : kk * e;
+    s.Kn[(cc * C + t) * Dk + x] = -kk * e;
+    sQ[t * LK + x] *= e;
+    sK[t * LK + x] = ke;
   }
   if (threadIdx.x == 0) s.dec[cc] = decay_exp(Gend);
   __syncthreads();
-  if (BWD) {
+  {
     float acc[4][NK];
     zero(acc);
     mm<4, NK, C, false, false>(acc, sT, LC, sK, LK);       // Y = (I + A)^-T Kend
@@ -276,18 +274,16 @@ gdn_prep_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __res
     zero(acc);
     mm<4, 2, C, true, false>(acc, sT, LC, sV, LV);
     each(acc, [&](int t, int x, float y) { s.U[(cc * C + t) * DvP + v0 + x] = y; });
-    if (BWD) {
-      __syncthreads();
-      load_rows<VS>(sV, LV, dO, d.Dv, v0, d.Dv - v0, d, bh, c);
-      __syncthreads();
-      zero(acc);
-      mm<4, 2, C, true, false>(acc, sA, LC, sV, LV);
-      each(acc, [&](int t, int x, float y) { s.X[(cc * C + t) * DvP + v0 + x] = y; });
-      float az[NK][2];
-      zero(az);
-      mm<NK, 2, C, false, false>(az, sQ, LK, sV, LV);
-      each(az, [&](int r, int x, float y) { s.Z[(cc * Dk + r) * DvP + v0 + x] = y; });
-    }
+    __syncthreads();
+    load_rows<VS>(sV, LV, dO, d.Dv, v0, d.Dv - v0, d, bh, c);
+    __syncthreads();
+    zero(acc);
+    mm<4, 2, C, true, false>(acc, sA, LC, sV, LV);
+    each(acc, [&](int t, int x, float y) { s.X[(cc * C + t) * DvP + v0 + x] = y; });
+    float az[NK][2];
+    zero(az);
+    mm<NK, 2, C, false, false>(az, sQ, LK, sV, LV);
+    each(az, [&](int r, int x, float y) { s.Z[(cc * Dk + r) * DvP + v0 + x] = y; });
   }
 }
 
@@ -363,43 +359,6 @@ gdn_scan_kernel(const float* __restrict__ M1, const float* __restrict__ M2, floa
     mm<NK, 2, C, false, false>(ns, t + C * LK, LK, sV, LV);
     each(ns, [&](int r, int x, float y) { St[r * LV + x] = e * St[r * LV + x] + y + (REV ? sZ[r * LV + x] : 0.f); });
     __syncthreads();
-  }
-}
-
-// ---------------------------------------------------------------------------------------------- forward output
-template <int Dk>
-constexpr int out_smem() { return (C * (Dk + 4) + C * LC + Dk * LV + C * LV + 2 * C) * 4; }
-
-template <int Dk, typename T, typename TO>
-__global__ void __launch_bounds__(kThreads)
-gdn_out_kernel(const T* __restrict__ q, const float* __restrict__ g, const float* __restrict__ beta, Scratch s, TO* __restrict__ o, Dims d) {
-  extern __shared__ __align__(16) float sm[];
-  constexpr int LK = Dk + 4;
-  float* sQ = sm;
-  float* sP = sQ + C * LK;
-  float* sS = sP + C * LC;
-  float* sR = sS + Dk * LV;
-  float* G = sR + C * LV;
-  float* bt = G + C;
-  const int c = blockIdx.x, bh = blockIdx.y;
-  const long cc = (long)bh * d.n + c;
-  const int DvP = (d.Dv + VS - 1) / VS * VS;
-  load_rows<Dk>(sQ, LK, q, Dk, 0, Dk, d, bh, c);
-  for (int i = threadIdx.x; i < C * C; i += kThreads) sP[(i / C) * LC + i % C] = s.P[cc * C * C + i];
-  load_gates(G, bt, g, beta, d, bh, c);
-  for (int i = threadIdx.x; i < C * Dk; i += kThreads) sQ[(i / Dk) * LK + i % Dk] *= decay_exp(G[i / Dk]);
-  for (int v0 = 0; v0 < d.Dv; v0 += VS) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < Dk * VS; i += kThreads) sS[(i / VS) * LV + i % VS] = s.S[(cc * Dk + i / VS) * DvP + v0 + i % VS];
-    for (int i = threadIdx.x; i < C * VS; i += kThreads) sR[(i / VS) * LV + i % VS] = s.U[(cc * C + i / VS) * DvP + v0 + i % VS];
-    __syncthreads();
-    float acc[4][2];
-    zero(acc);
-    mm<4, 2, Dk, true, false>(acc, sQ, LK, sS, LV);
-    mm<4, 2, C, true, false>(acc, sP, LC, sR, LV);
-    each(acc, [&](int t, int x, float y) {
-      if (c * C + t < d.T && v0 + x < d.Dv) put(o + in_row(d, bh, c, t) * d.Dv + v0 + x, y);
-    });
   }
 }
 
@@ -566,22 +525,20 @@ gdn_grads_kernel(const T* __restrict__ q, const T* __restrict__ k, const float* 
 }
 
 struct Layout {
-  long rk, rv, st, pp, cs;   // floats of a [rows x Dk], [rows x DvP], [chunks x Dk x DvP], [rows x 64], [chunks] array
+  long rk, rv, st, cs;   // floats of a [rows x Dk], [rows x DvP], [chunks x Dk x DvP], [chunks] array
   Layout(int B, int T, int H, int Dk, int Dv) {
     const long chunks = (long)B * H * ((T + C - 1) / C), DvP = (Dv + VS - 1) / VS * VS;
     rk = chunks * C * Dk;
     rv = chunks * C * DvP;
     st = chunks * Dk * DvP;
-    pp = chunks * C * C;
     cs = (chunks + 3) / 4 * 4;
   }
-  long total(bool bwd) const { return 2 * rk + rv + st + cs + (bwd ? 2 * rk + rv + 2 * st : pp); }
-  Scratch split(float* p, bool bwd) const {
-    Scratch s{};
+  long total() const { return 4 * rk + 2 * rv + 3 * st + cs; }
+  Scratch split(float* p) const {
     auto take = [&](long n) { float* r = p; p += n; return r; };
+    Scratch s{};
     s.W = take(rk); s.Ke = take(rk); s.U = take(rv); s.S = take(st); s.dec = take(cs);
-    if (bwd) { s.Y = take(rk); s.Kn = take(rk); s.X = take(rv); s.Z = take(st); s.dS = take(st); }
-    else s.P = take(pp);
+    s.Y = take(rk); s.Kn = take(rk); s.X = take(rv); s.Z = take(st); s.dS = take(st);
     return s;
   }
 };
@@ -592,34 +549,17 @@ bool allow_smem(K kernel, int bytes) {
 }
 
 template <int Dk, typename T>
-int run_fwd(const T* q, const T* k, const T* v, const float* g, const float* beta, __nv_bfloat16* o, float* scratch, int B, int T_, int H,
-            int Dv, cudaStream_t st) {
-  static const bool ok = allow_smem(gdn_prep_kernel<Dk, false, T>, prep_smem<Dk>()) && allow_smem(gdn_scan_kernel<Dk, false>, scan_smem<Dk>()) &&
-                         allow_smem(gdn_out_kernel<Dk, T, __nv_bfloat16>, out_smem<Dk>());
-  if (!ok) return -4;
-  const Layout l(B, T_, H, Dk, Dv);
-  const Scratch s = l.split(scratch, false);
-  const Dims d{T_, H, Dv, (T_ + C - 1) / C};
-  const int slices = (Dv + VS - 1) / VS;
-  const dim3 chunks(d.n, B * H), heads(B * H, slices);
-  gdn_prep_kernel<Dk, false, T><<<chunks, kThreads, prep_smem<Dk>(), st>>>(q, k, v, g, beta, nullptr, s, d);
-  gdn_scan_kernel<Dk, false><<<heads, kThreads, scan_smem<Dk>(), st>>>(s.W, s.Ke, s.U, nullptr, s.dec, s.S, d.n, slices * VS);
-  gdn_out_kernel<Dk, T, __nv_bfloat16><<<chunks, kThreads, out_smem<Dk>(), st>>>(q, g, beta, s, o, d);
-  return cudaGetLastError() == cudaSuccess ? 0 : -5;
-}
-
-template <int Dk, typename T>
 int run_bwd(const T* q, const T* k, const T* v, const float* g, const float* beta, const T* dO, T* dq, T* dk, T* dv, float* dg, float* dbeta,
             float* scratch, int B, int T_, int H, int Dv, cudaStream_t st) {
-  static const bool ok = allow_smem(gdn_prep_kernel<Dk, true, T>, prep_smem<Dk>()) && allow_smem(gdn_scan_kernel<Dk, false>, scan_smem<Dk>()) &&
+  static const bool ok = allow_smem(gdn_prep_kernel<Dk, T>, prep_smem<Dk>()) && allow_smem(gdn_scan_kernel<Dk, false>, scan_smem<Dk>()) &&
                          allow_smem(gdn_scan_kernel<Dk, true>, scan_smem<Dk>()) && allow_smem(gdn_grads_kernel<Dk, T>, grads_smem<Dk>());
   if (!ok) return -4;
   const Layout l(B, T_, H, Dk, Dv);
-  const Scratch s = l.split(scratch, true);
+  const Scratch s = l.split(scratch);
   const Dims d{T_, H, Dv, (T_ + C - 1) / C};
   const int slices = (Dv + VS - 1) / VS;
   const dim3 chunks(d.n, B * H), heads(B * H, slices);
-  gdn_prep_kernel<Dk, true, T><<<chunks, kThreads, prep_smem<Dk>(), st>>>(q, k, v, g, beta, dO, s, d);
+  gdn_prep_kernel<Dk, T><<<chunks, kThreads, prep_smem<Dk>(), st>>>(q, k, v, g, beta, dO, s, d);
   gdn_scan_kernel<Dk, false><<<heads, kThreads, scan_smem<Dk>(), st>>>(s.W, s.Ke, s.U, nullptr, s.dec, s.S, d.n, slices * VS);
   gdn_scan_kernel<Dk, true><<<heads, kThreads, scan_smem<Dk>(), st>>>(s.Y, s.Kn, s.X, s.Z, s.dec, s.dS, d.n, slices * VS);
   gdn_grads_kernel<Dk, T><<<chunks, kThreads, grads_smem<Dk>(), st>>>(q, k, g, beta, dO, s, dq, dk, dv, dg, dbeta, d);
@@ -635,22 +575,13 @@ int check(int B, int T, int H, int Dk, int Dv) {
 }  // namespace
 
 // Floats of scratch for one call (16-byte aligned buffer).
-extern "C" long long sr_gdn_chunk_scratch(int B, int T, int H, int Dk, int Dv, int bwd) {
+extern "C" long long sr_gdn_chunk_scratch(int B, int T, int H, int Dk, int Dv) {
   if (B <= 0 || T <= 0 || H <= 0 || Dk <= 0 || Dv <= 0) return 0;
-  return Layout(B, T, H, Dk, Dv).total(bwd != 0);
+  return Layout(B, T, H, Dk, Dv).total();
 }
 
-// q, k: bf16 [B, T, H, Dk]; v, o: bf16 [B, T, H, Dv]; g (log-decay <= 0), beta: fp32 [B, T, H]; all contiguous; Dk 64 or 128.
-extern "C" int sr_gdn_chunk_fwd(const void* q, const void* k, const void* v, const float* g, const float* beta, void* o, float* scratch,
-                                int B, int T, int H, int Dk, int Dv, cudaStream_t s) {
-  if (B <= 0 || T <= 0 || H <= 0) return 0;
-  if (int rc = check(B, T, H, Dk, Dv)) return rc;
-  using bf = __nv_bfloat16;
-  auto f = Dk == 64 ? run_fwd<64, bf> : run_fwd<128, bf>;
-  return f((const bf*)q, (const bf*)k, (const bf*)v, g, beta, (bf*)o, scratch, B, T, H, Dv, s);
-}
-
-// Gradients of the same call from dO. q, k, v, dO and dq, dk, dv: all bf16 or (fp32 != 0) all fp32; dg, dbeta fp32.
+// Gradients of o = gated_delta_rule(q, k, v, g, beta) from dO. q, k, dq, dk: [B, T, H, Dk]; v, dv, dO: [B, T, H, Dv], all bf16 or
+// (fp32 != 0) all fp32; g (log-decay), beta, dg, dbeta: fp32 [B, T, H]; all contiguous; Dk 64 or 128.
 extern "C" int sr_gdn_chunk_bwd(const void* q, const void* k, const void* v, const float* g, const float* beta, const void* dO, void* dq,
                                 void* dk, void* dv, float* dg, float* dbeta, float* scratch, int B, int T, int H, int Dk, int Dv, int fp32,
                                 cudaStream_t s) {

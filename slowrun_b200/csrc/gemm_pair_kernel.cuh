@@ -390,7 +390,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       tc_fence_before();
       mbar_arrive_cluster(tempty0 + buf * 8);
     }
-    if (lane == 0) bulk_wait_all();
+    if (lane == 0) bulk_wait_read<0>();   // the boxes must outlive their reads; the writes are done when the kernel is
   }
 
   // ------------------------------------------------------------ teardown

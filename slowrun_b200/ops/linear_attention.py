@@ -10,11 +10,11 @@ Attention). The reference fork delegates this to flash-linear-attention's Triton
 * `gated_delta_rule_chunked`    chunk-parallel form in plain PyTorch (differentiable, any device): inside a chunk the
                                 writes are obtained from one unit-lower-triangular solve, chunks are chained through
                                 the state. Every exponential is of a non-positive number, so it is safe for any decay;
-* `gated_delta_rule`            the op the model calls: on a GPU, with one decay per head, backward and (long
-                                sequences) forward run the chunked form as CUDA kernels (csrc/gated_delta_chunk.cu); other
-                                forwards run the CUDA recurrence (csrc/gated_delta.cu, state in registers), and the
-                                backward of per-channel decays re-derives the gradients from the PyTorch chunked form;
-                                elsewhere it is the chunked form throughout.
+* `gated_delta_rule`            the op the model calls: on a GPU, the forward runs the CUDA recurrence kernel
+                                (csrc/gated_delta.cu, state in registers). The backward with one decay per head runs the
+                                chunked form as CUDA kernels (csrc/gated_delta_chunk.cu), with a decay per channel it
+                                re-derives the gradients from the PyTorch chunked form; elsewhere it is the chunked form
+                                throughout.
 """
 from __future__ import annotations
 
@@ -107,18 +107,6 @@ def gated_delta_rule_chunked(q, k, v, g, beta, chunk_size=None, initial_state=No
     return (o, S) if return_state else o
 
 
-# Sequences from here on take the chunk kernels in the forward. Their three launches cost about 80 us (Dk 64) or 110 us
-# (Dk 128) however short the sequence, the recurrence 0.5 to 0.8 us per token: at T = 128 it is 66 / 69 against 82 / 115 us
-# (14 heads of 64 / 8 of 128), at T = 256 129 / 135 against 89 / 131 us.
-CHUNK_FWD_MIN_T = 256
-
-
-def _chunk_scratch(B, T, H, Dk, Dv, bwd, device):
-    from . import _lib
-    n = _lib.fn("sr_gdn_chunk_scratch", [_lib.c_int] * 6, _lib.c_ll)(B, T, H, Dk, Dv, int(bwd))
-    return torch.empty(n, dtype=torch.float32, device=device)
-
-
 def _cuda_forward(q, k, v, g, beta):
     from . import _lib
     B, T, H, Dk = q.shape
@@ -127,13 +115,6 @@ def _cuda_forward(q, k, v, g, beta):
     gf, bf = g.float().contiguous(), beta.float().contiguous()
     o = torch.empty((B, T, H, Dv), dtype=torch.bfloat16, device=q.device)
     P, I = _lib.c_void_p, _lib.c_int
-    if g.dim() == 3 and T >= CHUNK_FWD_MIN_T and B * H <= 65535:
-        scratch = _chunk_scratch(B, T, H, Dk, Dv, False, q.device)
-        rc = _lib.fn("sr_gdn_chunk_fwd", [P] * 7 + [I] * 5 + [P])(
-            qb.data_ptr(), kb.data_ptr(), vb.data_ptr(), gf.data_ptr(), bf.data_ptr(), o.data_ptr(), scratch.data_ptr(),
-            B, T, H, Dk, Dv, _lib.stream_ptr())
-        _lib.check_rc(rc, "sr_gdn_chunk_fwd")
-        return o.to(v.dtype)
     rc = _lib.fn("sr_gated_delta_fwd", [P] * 7 + [I] * 7 + [P])(
         qb.data_ptr(), kb.data_ptr(), vb.data_ptr(), gf.data_ptr(), bf.data_ptr(), o.data_ptr(), 0, B, T, H, Dk, Dv,
         int(g.dim() == 4), 0, _lib.stream_ptr())
@@ -152,8 +133,9 @@ def _cuda_backward(q, k, v, g, beta, do):
     gf, bf = g.float().contiguous(), beta.float().contiguous()
     dq, dk, dv = torch.empty_like(qc), torch.empty_like(kc), torch.empty_like(vc)
     dg, db = torch.empty_like(gf), torch.empty_like(bf)
-    scratch = _chunk_scratch(B, T, H, Dk, Dv, True, q.device)
     P, I = _lib.c_void_p, _lib.c_int
+    n = _lib.fn("sr_gdn_chunk_scratch", [I] * 5, _lib.c_ll)(B, T, H, Dk, Dv)
+    scratch = torch.empty(n, dtype=torch.float32, device=q.device)
     rc = _lib.fn("sr_gdn_chunk_bwd", [P] * 12 + [I] * 6 + [P])(
         qc.data_ptr(), kc.data_ptr(), vc.data_ptr(), gf.data_ptr(), bf.data_ptr(), dc.data_ptr(), dq.data_ptr(), dk.data_ptr(),
         dv.data_ptr(), dg.data_ptr(), db.data_ptr(), scratch.data_ptr(), B, T, H, Dk, Dv, int(dt == torch.float32),
