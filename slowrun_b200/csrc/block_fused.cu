@@ -47,9 +47,9 @@ __device__ __forceinline__ void st2(__nv_bfloat16* p, float a, float b) {
 // ---------------------------------------------------------------------------------------------- per-head vectors
 // The kernels below work on (token, head) vectors of 128 elements. Eight lanes hold one: lane l has elements 8l .. 8l+7 and
 // 64+8l .. 64+8l+7, i.e. both partners of its rotary pairs, in two 16-byte accesses per tensor. A warp then has four vectors
-// in flight and a reduction is three shuffles; with a warp per vector it was five shuffles and 4-byte accesses for one, and
+// in flight and a reduction is six or twelve shuffles for four; with a warp per vector it was five shuffles and 4-byte accesses for one each, and
 // the kernels were bound by instructions. us, warp per vector -> this, [8192, 20 heads]: qkv_prep fwd 76 -> 50, bwd 114 -> 86,
-// attn_post bwd 57 -> 37; [65536, 8 heads]: 217 -> 152, 342 -> 293, 272 -> 195, attn_post fwd 101 -> 65.
+// attn_post bwd 57 -> 37; [65536, 8 heads]: 217 -> 158, 342 -> 293, 272 -> 187, attn_post fwd 101 -> 67.
 constexpr int kVecPerBlock = kThreads / 8;
 
 struct Vec {
@@ -88,12 +88,6 @@ __device__ __forceinline__ void stv(__nv_bfloat16* p, int l, const Vec& v) {
   st8(p + 8 * l, v.lo);
   st8(p + 64 + 8 * l, v.hi);
 }
-__device__ __forceinline__ float dot(const Vec& a, const Vec& b) {
-  float s = 0.f;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) s += a.lo[i] * b.lo[i] + a.hi[i] * b.hi[i];
-  return s;
-}
 // sum over the eight lanes of a vector
 __device__ __forceinline__ float sum8(float v) {
 #pragma unroll
@@ -101,15 +95,14 @@ __device__ __forceinline__ float sum8(float v) {
   return v;
 }
 
-// The forward kernels sum in the order of a butterfly over 32 lanes, so that their results do not depend on how many lanes
-// share a vector: a change of rounding in the forward travels through every later layer and shows as 1 to 2 % in gradients
-// that are sums with cancellation. Lane l stands for lanes 4l .. 4l+3 of a warp with elements {2L, 2L+1, 64+2L, 64+2L+1} each
-// (sum_sq_pairs) or for lanes 2l, 2l+1, 16+2l, 16+2l+1 with elements 4L .. 4L+3 (dot_quads).
-__device__ __forceinline__ float sum_sq_pairs(const Vec& o) {
+// The sums keep the order of a butterfly over 32 lanes, so that results do not depend on how many lanes share a vector: a
+// change of rounding travels through every later layer and shows as 1 to 2 % in gradients that are sums with cancellation. Lane l stands for lanes 4l .. 4l+3 of a warp with elements {2L, 2L+1, 64+2L, 64+2L+1} each
+// (dot_pairs) or for lanes 2l, 2l+1, 16+2l, 16+2l+1 with elements 4L .. 4L+3 (dot_quads).
+__device__ __forceinline__ float dot_pairs(const Vec& a, const Vec& b) {
   float s[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j)
-    s[j] = o.lo[2 * j] * o.lo[2 * j] + o.lo[2 * j + 1] * o.lo[2 * j + 1] + o.hi[2 * j] * o.hi[2 * j] + o.hi[2 * j + 1] * o.hi[2 * j + 1];
+    s[j] = a.lo[2 * j] * b.lo[2 * j] + a.lo[2 * j + 1] * b.lo[2 * j + 1] + a.hi[2 * j] * b.hi[2 * j] + a.hi[2 * j + 1] * b.hi[2 * j + 1];
 #pragma unroll
   for (int j = 0; j < 4; ++j) s[j] = sum8(s[j]);
   return (s[0] + s[2]) + (s[1] + s[3]);
@@ -161,7 +154,7 @@ qkv_prep_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* 
       o.lo[i] = x[which].lo[i] * c[i] + x[which].hi[i] * s[i];
       o.hi[i] = -x[which].lo[i] * s[i] + x[which].hi[i] * c[i];
     }
-    const float r = rsqrtf(sum_sq_pairs(o) * (1.f / 128.f) + eps);
+    const float r = rsqrtf(dot_pairs(o, o) * (1.f / 128.f) + eps);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       o.lo[i] *= r;
@@ -230,8 +223,8 @@ qkv_prep_bwd_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* 
       o.lo[i] = x.lo[i] * c[i] + x.hi[i] * s[i];
       o.hi[i] = -x.lo[i] * s[i] + x.hi[i] * c[i];
     }
-    const float r = rsqrtf(sum_sq_pairs(o) * (1.f / 128.f) + eps);
-    const float k = r * r * r * sum8(dot(o, g)) * (1.f / 128.f);
+    const float r = rsqrtf(dot_pairs(o, o) * (1.f / 128.f) + eps);
+    const float k = r * r * r * dot_pairs(o, g) * (1.f / 128.f);
     Vec w;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -254,7 +247,7 @@ qkv_prep_bwd_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* 
   if (ve != nullptr) {
     const float gt = gate[vid];
     const Vec e = ldv(ve + (long)tok * d + h * 128, l);
-    const float dg = sum8(dot(g, e));
+    const float dg = dot_quads(g, e);
     if (valid) {
       if (l == 0) dgate[vid] = dg;
 #pragma unroll

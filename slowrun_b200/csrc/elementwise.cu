@@ -645,31 +645,15 @@ __global__ void norm_bwd_drop_kernel(const __nv_bfloat16* __restrict__ x_mid, co
 
 // ------------------------------------------------------------------ the same four row kernels, a row in registers
 // The kernels above walk a row twice: at D = 2560 ten dependent steps of 16-byte loads per pass, with 8192 rows filling less
-// than one wave. Here a row sits in the registers of the threads that own it: every load is in flight at once and each input
-// is read once. The backward kernels use TPR threads per row (VPT vectors of 8 each) and blocks that walk over rows, so the
-// scalar sums of norm_bwd_mix cost three atomics per block and not per eight rows.
-// ROWS_MEASURED_PLACEHOLDER
+// than one wave. Here the row sits in the registers of its warp (VPT vectors of 8 per lane): the loads are in flight at once and
+// what the reduction needs is read once. One warp per row as above keeps the order of the sums, bit for bit: a change of
+// rounding travels through every later layer and shows as 1 to 2 % in gradients that are sums with cancellation (128 threads
+// per row measured a little faster and was not kept for that).
+// us, two walks -> these: [8192, 2560] norm_bwd_drop 72 -> 70, mix_norm_fwd 48 -> 30, add_norm_fwd 50 -> 48 (the dropout hash
+// bounds the two with a mask); [65536, 1024] norm_bwd_mix 247 -> 226, norm_bwd_drop 182 -> 145, mix_norm_fwd 129 -> 88,
+// add_norm_fwd 129 -> 126.
 constexpr int kRowThreads = 128;
 
-// sums of a and b over the TPR threads of a row; `red` holds 2 x 4 pairs that alternate, so one barrier per call suffices
-template <int TPR>
-__device__ __forceinline__ float2 group_sum(float a, float b, float2 (&red)[2][4], int& turn) {
-  a = warp_sum(a);
-  b = warp_sum(b);
-  const int warp = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) red[turn][warp] = make_float2(a, b);
-  __syncthreads();
-  constexpr int W = TPR / 32;
-  const int w0 = warp / W * W;
-  float2 r = red[turn][w0];
-#pragma unroll
-  for (int i = 1; i < W; ++i) {
-    r.x += red[turn][w0 + i].x;
-    r.y += red[turn][w0 + i].y;
-  }
-  turn ^= 1;
-  return r;
-}
 __device__ __forceinline__ void unpack8(const uint4& t, float (&f)[8]) {
   const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&t);
 #pragma unroll
@@ -688,25 +672,17 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 }
 __device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16(x)); }
 
-// f(row, valid) for the rows of this group; all threads of the block make the same number of steps
-#define SR_FOR_ROWS(TPR)                                                                                    \
-  constexpr int RPB = kRowThreads / (TPR);                                                                  \
-  const int tid = threadIdx.x % (TPR);                                                                      \
-  for (long row0 = (long)blockIdx.x * RPB; row0 < rows; row0 += (long)gridDim.x * RPB)
-
-template <int TPR, int VPT, typename F>
-__device__ __forceinline__ void row_vectors(int tid, int D, bool valid, F f) {
+// f(i, column) for the vectors of a row that this lane owns
+template <int VPT, typename F>
+__device__ __forceinline__ void row_vectors(int lane, int D, F f) {
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
-    const int c = (tid + i * TPR) * 8;
-    if (valid && c < D) f(i, c);
+    const int c = (lane + i * 32) * 8;
+    if (c < D) f(i, c);
   }
 }
 #define LDV(p) (*reinterpret_cast<const uint4*>(p))
 
-// The two forward kernels keep one warp per row (VPT vectors per lane, all in flight at once): their sum of squares is then
-// taken in the order of the kernels above, bit for bit. A change of rounding in the forward would travel through every later
-// layer and show as 1 to 2 % in gradients that are sums with cancellation.
 template <int VPT>
 __global__ void __launch_bounds__(kRowThreads)
 mix_norm_fwd_rows(const __nv_bfloat16* __restrict__ xp, const __nv_bfloat16* __restrict__ x0, const __nv_bfloat16* __restrict__ skip,
@@ -718,13 +694,13 @@ mix_norm_fwd_rows(const __nv_bfloat16* __restrict__ xp, const __nv_bfloat16* __r
   const float lr = *lr_p, l0 = *l0_p, ws = skip ? *ws_p : 0.f;
   const long base = row * (long)D;
   uint4 A[VPT], B[VPT], S[VPT];
-  row_vectors<32, VPT>(lane, D, true, [&](int i, int c) {
+  row_vectors<VPT>(lane, D, [&](int i, int c) {
     A[i] = LDV(xp + base + c);
     B[i] = LDV(x0 + base + c);
     if (skip) S[i] = LDV(skip + base + c);
   });
   float ss = 0.f;
-  row_vectors<32, VPT>(lane, D, true, [&](int i, int c) {
+  row_vectors<VPT>(lane, D, [&](int i, int c) {
     float a[8], b[8];
     unpack8(A[i], a);
     unpack8(B[i], b);
@@ -744,7 +720,7 @@ mix_norm_fwd_rows(const __nv_bfloat16* __restrict__ xp, const __nv_bfloat16* __r
   });
   ss = warp_sum(ss);
   const float r = rsqrtf(ss / D + eps);
-  row_vectors<32, VPT>(lane, D, true, [&](int i, int c) {
+  row_vectors<VPT>(lane, D, [&](int i, int c) {
     float f[8];
     unpack8(A[i], f);
 #pragma unroll
@@ -766,12 +742,12 @@ add_norm_fwd_rows(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
   const uint32_t thr = keep_threshold(p);
   const long base = row * (long)D;
   uint4 A[VPT], B[VPT];
-  row_vectors<32, VPT>(lane, D, true, [&](int i, int c) {
+  row_vectors<VPT>(lane, D, [&](int i, int c) {
     A[i] = LDV(x + base + c);
     B[i] = LDV(y + base + c);
   });
   float ss = 0.f;
-  row_vectors<32, VPT>(lane, D, true, [&](int i, int c) {
+  row_vectors<VPT>(lane, D, [&](int i, int c) {
     float a[8], b[8];
     unpack8(A[i], a);
     unpack8(B[i], b);
@@ -786,7 +762,7 @@ add_norm_fwd_rows(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
   });
   ss = warp_sum(ss);
   const float r = rsqrtf(ss / D + eps);
-  row_vectors<32, VPT>(lane, D, true, [&](int i, int c) {
+  row_vectors<VPT>(lane, D, [&](int i, int c) {
     float f[8];
     unpack8(A[i], f);
 #pragma unroll
@@ -795,59 +771,57 @@ add_norm_fwd_rows(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
   });
 }
 
-template <int TPR, int VPT>
+template <int VPT>
 __global__ void __launch_bounds__(kRowThreads)
 norm_bwd_drop_rows(const __nv_bfloat16* __restrict__ x_mid, const __nv_bfloat16* __restrict__ dn, const __nv_bfloat16* __restrict__ g_res,
                    __nv_bfloat16* __restrict__ dx_mid, __nv_bfloat16* __restrict__ dy, long rows, int D, float eps, float p,
                    uint64_t salt, const unsigned long long* __restrict__ seed_ptr) {
-  __shared__ float2 red[2][4];
-  int turn = 0;
+  const long row = (long)blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const int lane = threadIdx.x & 31;
   const uint64_t seed = salt + (seed_ptr ? (*seed_ptr) * 0x9E3779B97F4A7C15ull : 0ull);
   const float scale = 1.f / (1.f - p);
   const uint32_t thr = keep_threshold(p);
-  SR_FOR_ROWS(TPR) {
-    const long row = row0 + threadIdx.x / TPR;
-    const bool valid = row < rows;
-    const long base = row * (long)D;
-    uint4 X[VPT], G[VPT], R[VPT];
-    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
-      X[i] = LDV(x_mid + base + c);
-      G[i] = LDV(dn + base + c);
-      R[i] = LDV(g_res + base + c);
-    });
-    float ss = 0.f, dot = 0.f;
-    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int) {
-      float f[8], g[8];
-      unpack8(X[i], f);
-      unpack8(G[i], g);
+  const long base = row * (long)D;
+  uint4 X[VPT], G[VPT], R[VPT];
+  row_vectors<VPT>(lane, D, [&](int i, int c) {
+    X[i] = LDV(x_mid + base + c);
+    G[i] = LDV(dn + base + c);
+    R[i] = LDV(g_res + base + c);
+  });
+  float ss = 0.f, dot = 0.f;
+  row_vectors<VPT>(lane, D, [&](int i, int) {
+    float f[8], g[8];
+    unpack8(X[i], f);
+    unpack8(G[i], g);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        ss += f[j] * f[j];
-        dot += f[j] * g[j];
-      }
-    });
-    const float2 t = group_sum<TPR>(ss, dot, red, turn);
-    const float r = rsqrtf(t.x / D + eps);
-    const float k = r * r * r * t.y / D;
-    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
-      float f[8], g[8], a[8], o[8], d[8];
-      unpack8(X[i], f);
-      unpack8(G[i], g);
-      unpack8(R[i], a);
+    for (int j = 0; j < 8; ++j) {
+      ss += f[j] * f[j];
+      dot += f[j] * g[j];
+    }
+  });
+  ss = warp_sum(ss);
+  dot = warp_sum(dot);
+  const float r = rsqrtf(ss / D + eps);
+  const float k = r * r * r * dot / D;
+  row_vectors<VPT>(lane, D, [&](int i, int c) {
+    float f[8], g[8], a[8], o[8], d[8];
+    unpack8(X[i], f);
+    unpack8(G[i], g);
+    unpack8(R[i], a);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = round_bf16(r * g[j] - k * f[j] + a[j]);
-      store8(dx_mid + base + c, o);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const bool keep = (p > 0.f) ? keep_elem(seed, (uint64_t)(base + c + j), thr) : true;
-        d[j] = keep ? scale * o[j] : 0.f;
-      }
-      store8(dy + base + c, d);
-    });
-  }
+    for (int j = 0; j < 8; ++j) {
+      o[j] = round_bf16(r * g[j] - k * f[j] + a[j]);
+      const bool keep = (p > 0.f) ? keep_elem(seed, (uint64_t)(base + c + j), thr) : true;
+      d[j] = keep ? scale * o[j] : 0.f;
+    }
+    store8(dx_mid + base + c, o);
+    store8(dy + base + c, d);
+  });
 }
 
-template <int TPR, int VPT>
+// Blocks walk over rows, so the scalar sums cost three atomics per block and not per eight rows.
+template <int VPT>
 __global__ void __launch_bounds__(kRowThreads)
 norm_bwd_mix_rows(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ da, const __nv_bfloat16* __restrict__ g_res,
                   const __nv_bfloat16* __restrict__ g_res2, const __nv_bfloat16* __restrict__ xp, const __nv_bfloat16* __restrict__ x0,
@@ -855,27 +829,19 @@ norm_bwd_mix_rows(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
                   __nv_bfloat16* __restrict__ dskip, const float* __restrict__ lr_p, const float* __restrict__ l0_p,
                   const float* __restrict__ ws_p, float* __restrict__ d_lr, float* __restrict__ d_l0, float* __restrict__ d_ws,
                   long rows, int D, float eps) {
-  __shared__ float2 red[2][4];
-  __shared__ float red1[32];
-  int turn = 0;
+  __shared__ float red[32];
+  const int lane = threadIdx.x & 31;
   const float lr = *lr_p, l0 = *l0_p, ws = skip ? *ws_p : 0.f;
   float s_lr = 0.f, s_l0 = 0.f, s_ws = 0.f;
-  SR_FOR_ROWS(TPR) {
-    const long row = row0 + threadIdx.x / TPR;
-    const bool valid = row < rows;
+  for (long row = (long)blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5); row < rows; row += (long)gridDim.x * (kRowThreads / 32)) {
     const long base = row * (long)D;
-    uint4 X[VPT], G[VPT], R[VPT], R2[VPT], A[VPT], B[VPT], S[VPT];
-    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
+    uint4 X[VPT], G[VPT];
+    row_vectors<VPT>(lane, D, [&](int i, int c) {
       X[i] = LDV(x + base + c);
       G[i] = LDV(da + base + c);
-      R[i] = LDV(g_res + base + c);
-      if (g_res2) R2[i] = LDV(g_res2 + base + c);
-      A[i] = LDV(xp + base + c);
-      B[i] = LDV(x0 + base + c);
-      if (skip) S[i] = LDV(skip + base + c);
     });
     float ss = 0.f, dot = 0.f;
-    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int) {
+    row_vectors<VPT>(lane, D, [&](int i, int) {
       float f[8], g[8];
       unpack8(X[i], f);
       unpack8(G[i], g);
@@ -885,27 +851,28 @@ norm_bwd_mix_rows(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
         dot += f[j] * g[j];
       }
     });
-    const float2 t = group_sum<TPR>(ss, dot, red, turn);
-    const float r = rsqrtf(t.x / D + eps);
-    const float k = r * r * r * t.y / D;
-    row_vectors<TPR, VPT>(tid, D, valid, [&](int i, int c) {
+    ss = warp_sum(ss);
+    dot = warp_sum(dot);
+    const float r = rsqrtf(ss / D + eps);
+    const float k = r * r * r * dot / D;
+    row_vectors<VPT>(lane, D, [&](int i, int c) {
       float f[8], g[8], e[8], a[8], b[8], o[8];
       unpack8(X[i], f);
       unpack8(G[i], g);
-      unpack8(R[i], e);
+      load8(g_res + base + c, e);
       if (g_res2) {   // second residual gradient (the stochastic-depth bypass), added in bf16 like a separate add would
         float e2[8];
-        unpack8(R2[i], e2);
+        load8(g_res2 + base + c, e2);
 #pragma unroll
         for (int j = 0; j < 8; ++j) e[j] = round_bf16(e[j] + e2[j]);
       }
-      unpack8(A[i], a);
-      unpack8(B[i], b);
+      load8(xp + base + c, a);
+      load8(x0 + base + c, b);
 #pragma unroll
       for (int j = 0; j < 8; ++j) g[j] = round_bf16(r * g[j] - k * f[j] + e[j]);
       if (skip) {
         float sk[8];
-        unpack8(S[i], sk);
+        load8(skip + base + c, sk);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           a[j] += ws * sk[j];
@@ -926,9 +893,9 @@ norm_bwd_mix_rows(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
       store8(dx0 + base + c, o);
     });
   }
-  s_lr = block_sum(s_lr, red1);
-  s_l0 = block_sum(s_l0, red1);
-  s_ws = block_sum(s_ws, red1);
+  s_lr = block_sum(s_lr, red);
+  s_l0 = block_sum(s_l0, red);
+  s_ws = block_sum(s_ws, red);
   if (threadIdx.x == 0) {
     atomicAdd(d_lr, s_lr);
     atomicAdd(d_l0, s_l0);
@@ -966,32 +933,23 @@ inline int grid_for(long n, int per_block) {
 }
 inline int rc() { return cudaGetLastError() == cudaSuccess ? 0 : -5; }
 
-// The backward kernels: rows of 264 to 4096 elements, 64 threads up to 512, 128 beyond, as many vectors per thread as the row
-// needs. Shorter rows are one step for a warp as it is, longer ones would not fit the registers.
-template <typename F>
-bool row_dispatch(int D, F f) {
-  if (D <= 256 || D > 4096) return false;
-  if (D <= 512) f(std::integral_constant<int, 64>(), std::integral_constant<int, 1>());
-  else if (D <= 1024) f(std::integral_constant<int, 128>(), std::integral_constant<int, 1>());
-  else if (D <= 2048) f(std::integral_constant<int, 128>(), std::integral_constant<int, 2>());
-  else if (D <= 3072) f(std::integral_constant<int, 128>(), std::integral_constant<int, 3>());
-  else f(std::integral_constant<int, 128>(), std::integral_constant<int, 4>());
-  return true;
-}
-// The forward kernels: one warp per row, vectors per lane = ceil(D / 256) up to 10 (longer rows would not fit the registers).
+// Vectors per lane = ceil(D / 256), 2 to V: shorter rows are one step for a warp as it is, longer ones would not fit the
+// registers; both take the kernels above. V is 10, and 4 for norm_bwd_mix, whose five to seven inputs leave too few loads in
+// flight at ten vectors: [8192, 2560] took 124 us against 110 of the kernel above, [65536, 1024] 226 against 247.
 template <int V, typename F>
-bool row_dispatch_warp(int D, F f) {
+bool row_dispatch(int D, F f) {
   if (D <= 256 || D > 256 * V) return false;
   if (D > 256 * (V - 1)) {
     f(std::integral_constant<int, V>());
     return true;
   }
-  if constexpr (V > 2) return row_dispatch_warp<V - 1>(D, f);
+  if constexpr (V > 2) return row_dispatch<V - 1>(D, f);
   return false;
 }
-inline unsigned row_grid(long rows, int tpr, int blocks_per_sm) {
-  const long b = (rows * tpr + kRowThreads - 1) / kRowThreads, cap = (long)sm_count() * blocks_per_sm;
-  return (unsigned)(b < cap ? b : cap);
+// one warp per row; `per_sm` > 0 caps the blocks
+inline unsigned row_grid(long rows, int per_sm) {
+  const long b = (rows + kRowThreads / 32 - 1) / (kRowThreads / 32), cap = (long)sm_count() * per_sm;
+  return (unsigned)(per_sm > 0 && b > cap ? cap : b);
 }
 
 }  // namespace
@@ -1096,8 +1054,8 @@ extern "C" int sr_add_norm_fwd(const void* x, const void* y, void* x_mid, void* 
                                unsigned long long seed, const unsigned long long* seed_ptr, cudaStream_t s) {
   if (D % 8) return -2;
   if (rows <= 0) return 0;
-  if (row_dispatch_warp<10>(D, [&](auto vpt) {
-        add_norm_fwd_rows<vpt.value><<<(unsigned)((rows + kRowThreads / 32 - 1) / (kRowThreads / 32)), kRowThreads, 0, s>>>(
+  if (row_dispatch<10>(D, [&](auto vpt) {
+        add_norm_fwd_rows<vpt.value><<<row_grid(rows, 0), kRowThreads, 0, s>>>(
             BF(x), BF(y), BFM(x_mid), BFM(n), rows, D, eps, p, seed, seed_ptr);
       }))
     return rc();
@@ -1111,8 +1069,8 @@ extern "C" int sr_norm_bwd_drop(const void* x_mid, const void* dn, const void* g
                                 cudaStream_t s) {
   if (D % 8) return -2;
   if (rows <= 0) return 0;
-  if (row_dispatch(D, [&](auto tpr, auto vpt) {
-        norm_bwd_drop_rows<tpr.value, vpt.value><<<row_grid(rows, tpr.value, 64), kRowThreads, 0, s>>>(
+  if (row_dispatch<10>(D, [&](auto vpt) {
+        norm_bwd_drop_rows<vpt.value><<<row_grid(rows, 0), kRowThreads, 0, s>>>(
             BF(x_mid), BF(dn), BF(g_res), BFM(dx_mid), BFM(dy), rows, D, eps, p, seed, seed_ptr);
       }))
     return rc();
@@ -1126,8 +1084,8 @@ extern "C" int sr_mix_norm_fwd(const void* xp, const void* x0, const void* skip,
                                const float* l0, const float* ws, long rows, int D, float eps, cudaStream_t s) {
   if (D % 8) return -2;
   if (rows <= 0) return 0;
-  if (row_dispatch_warp<10>(D, [&](auto vpt) {
-        mix_norm_fwd_rows<vpt.value><<<(unsigned)((rows + kRowThreads / 32 - 1) / (kRowThreads / 32)), kRowThreads, 0, s>>>(
+  if (row_dispatch<10>(D, [&](auto vpt) {
+        mix_norm_fwd_rows<vpt.value><<<row_grid(rows, 0), kRowThreads, 0, s>>>(
             BF(xp), BF(x0), BF(skip), BFM(x), BFM(a), lr, l0, ws, rows, D, eps);
       }))
     return rc();
@@ -1145,8 +1103,8 @@ extern "C" int sr_norm_bwd_mix(const void* x, const void* da, const void* g_res,
                                cudaStream_t s) {
   if (D % 8) return -2;
   if (rows <= 0) return 0;
-  if (row_dispatch(D, [&](auto tpr, auto vpt) {
-        norm_bwd_mix_rows<tpr.value, vpt.value><<<row_grid(rows, tpr.value, 8), kRowThreads, 0, s>>>(
+  if (row_dispatch<4>(D, [&](auto vpt) {
+        norm_bwd_mix_rows<vpt.value><<<row_grid(rows, 16), kRowThreads, 0, s>>>(
             BF(x), BF(da), BF(g_res), BF(g_res2), BF(xp), BF(x0), BF(skip), BFM(dxp), BFM(dx0), BFM(dskip), lr, l0, ws, d_lr,
             d_l0, d_ws, rows, D, eps);
       }))

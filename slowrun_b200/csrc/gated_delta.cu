@@ -23,16 +23,9 @@ namespace {
 constexpr int kChan = 2;           // value channels per warp
 constexpr int kWarpsPerBlock = 4;
 
-static_assert(kChan == 2, "the reductions below take the two channels of a warp together");
-
-// Sums of a and b over the warp: lanes 0..15 receive that of a, lanes 16..31 that of b. Five shuffles for both (the first one
-// swaps halves) in the order of a butterfly 16, 8, 4, 2, 1; one butterfly each would be ten, and shuffles are the largest part
-// of what a token issues: GD_MEASURED_PLACEHOLDER
-__device__ __forceinline__ float warp_sum_pair(float a, float b, int lane) {
-  const bool low = lane < 16;
-  float v = (low ? a : b) + __shfl_xor_sync(0xffffffffu, low ? b : a, 16);
+__device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
-  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
@@ -98,12 +91,8 @@ gated_delta_fwd_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
       }
       u[c] = a;
     }
-    {
-      const float mine = warp_sum_pair(u[0], u[1], lane);
-      const float other = __shfl_xor_sync(0xffffffffu, mine, 16);
-      u[0] = lane < 16 ? mine : other;
-      u[1] = lane < 16 ? other : mine;
-    }
+#pragma unroll
+    for (int c = 0; c < kChan; ++c) u[c] = warp_sum(u[c]);
     float out[kChan];
 #pragma unroll
     for (int c = 0; c < kChan; ++c) {
@@ -116,8 +105,14 @@ gated_delta_fwd_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
       }
       out[c] = a;
     }
-    const float o_mine = warp_sum_pair(out[0], out[1], lane);
-    if ((lane & 15) == 0 && c0 + (lane >> 4) < Dv) o[((tok0 + t) * H + h) * Dv + c0 + (lane >> 4)] = __float2bfloat16(o_mine);
+#pragma unroll
+    for (int c = 0; c < kChan; ++c) out[c] = warp_sum(out[c]);
+    if (lane == 0) {
+      const long row = (tok0 + t) * H + h;
+#pragma unroll
+      for (int c = 0; c < kChan; ++c)
+        if (c0 + c < Dv) o[row * Dv + c0 + c] = __float2bfloat16(out[c]);
+    }
     if (t + 1 < T) {
 #pragma unroll
       for (int i = 0; i < KPL; ++i) {
