@@ -47,9 +47,9 @@ __device__ __forceinline__ void st2(__nv_bfloat16* p, float a, float b) {
 // ---------------------------------------------------------------------------------------------- per-head vectors
 // The kernels below work on (token, head) vectors of 128 elements. Eight lanes hold one: lane l has elements 8l .. 8l+7 and
 // 64+8l .. 64+8l+7, i.e. both partners of its rotary pairs, in two 16-byte accesses per tensor. A warp then has four vectors
-// in flight and a reduction is six or twelve shuffles for four; with a warp per vector it was five shuffles and 4-byte accesses for one each, and
-// the kernels were bound by instructions. us, warp per vector -> this, [8192, 20 heads]: qkv_prep fwd 76 -> 50, bwd 114 -> 86,
-// attn_post bwd 57 -> 37; [65536, 8 heads]: 217 -> 158, 342 -> 293, 272 -> 187, attn_post fwd 101 -> 67.
+// in flight and a reduction is six or twelve shuffles for the four of them; with a warp per vector it was five shuffles each
+// and 4-byte accesses, and the kernels were bound by instructions. us, warp per vector -> this, [8192, 20 heads]: qkv_prep fwd
+// 76 -> 50, bwd 114 -> 88, attn_post bwd 57 -> 37; [65536, 8 heads]: 217 -> 158, 342 -> 293, 272 -> 187, attn_post fwd 101 -> 67.
 constexpr int kVecPerBlock = kThreads / 8;
 
 struct Vec {
