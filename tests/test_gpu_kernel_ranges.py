@@ -133,3 +133,76 @@ def test_gated_delta_chunk_kernels(T, Dk, Dv, decay):
     assert _rel(o, ref.detach()) < 4e-3
     for x, y in zip(grads, refs):
         assert (x.double() - y).norm().item() < 2e-5 * y.norm().item() + 1e-12
+
+
+# --------------------------------------------------------------------------------------------- logits and distillation
+@pytest.mark.parametrize("M,V,T,smoothing", [(1, 7, 0.5, 0.0), (5, 33, 1.0, 0.2), (64, 1000, 3.0, 0.0), (7, 50257, 1.0, 0.1)])
+def test_distillation_terms(M, V, T, smoothing):
+    """fp32 kernels against fp64: exponentials good to 2e-7 in sums of V terms."""
+    import torch.nn.functional as F
+    from slowrun_b200.ops import functional as ops
+    g = torch.Generator(device="cuda").manual_seed(V)
+    s, t = (3 * torch.randn(M, V, device="cuda", generator=g) for _ in range(2))
+    y = torch.randint(0, V, (M,), device="cuda", generator=g)
+    if M > 3:
+        y[1] = -1
+    a, b = s.clone().requires_grad_(), s.double().requires_grad_()
+    ce, kl = ops.distill_terms(a, t, y, T, smoothing)
+    grad, = torch.autograd.grad(0.3 * ce + 0.7 * kl, a)
+    keep = y != -1
+    ce64 = F.cross_entropy(b, y, label_smoothing=smoothing, ignore_index=-1)
+    kl64 = F.kl_div(F.log_softmax(b[keep] / T, -1), F.log_softmax(t.double()[keep] / T, -1), reduction="batchmean", log_target=True)
+    want, = torch.autograd.grad(0.3 * ce64 + 0.7 * kl64, b)
+    assert _rel(ce.detach(), ce64.detach()) < 2e-6 and _rel(kl.detach(), kl64.detach()) < 4e-6 and _rel(grad, want) < 4e-6
+
+
+@pytest.mark.parametrize("cap,vocab", [(15.0, 1001), (0.0, 1001), (10.0, 1008)])
+def test_softcapped_logits(cap, vocab):
+    from slowrun_b200.ops import functional as ops
+    g = torch.Generator(device="cuda").manual_seed(vocab)
+    x = (8 * torch.randn(3, 5, 1008, device="cuda", generator=g)).bfloat16()
+    x[0, 0, :4] = torch.tensor([0.0, 1e-3, 300.0, -300.0])
+    a, b = x.clone().requires_grad_(), x.double().requires_grad_()
+    z, zr = ops._softcap_logits(a, cap, vocab), b[..., :vocab]
+    zr = cap * torch.tanh(zr / cap) if cap > 0 else zr
+    w = torch.randn(z.shape, device="cuda", generator=g)
+    grad, = torch.autograd.grad(z, a, w)
+    want, = torch.autograd.grad(zr, b, w.double())
+    assert z.is_contiguous() and z.dtype == torch.float32
+    assert _rel(z.detach(), zr.detach()) < 3e-7 and _rel(grad, want) < 4e-3          # fp32; bf16 gradient
+
+
+# --------------------------------------------------------------------------------------------- block in one host call
+@pytest.mark.parametrize("track,T", [("limited", 200), ("two_hour", 256), ("tiny", 328)])
+def test_block_in_one_host_call_equals_the_calls_one_by_one(track, T, monkeypatch):
+    """Same launches in the same order: losses agree to the bit, gradients up to the order of split-K and dQ additions, which
+    differs between two runs of either path."""
+    from slowrun_b200.config import track_defaults
+    from slowrun_b200.models.gpt import build_model
+    from slowrun_b200.ops import block as block_ops, functional as ops
+    cfg = track_defaults(track)
+    m = cfg.model
+    m.n_layer, m.n_embd, m.n_head, m.n_kv_head, m.sequence_len = 4, 384, 3, 3, T
+    model = build_model(m, torch.device("cuda"), seed=0)
+    with torch.no_grad():
+        for p in model.parameters():
+            if not bool((p != 0).any()):
+                p.normal_(0.0, 0.02)
+    model.arena.refresh_shadows()
+    idx = torch.randint(0, 50257, (2, T + 1), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    results = []
+    for one_call in (True, False):
+        if not one_call:
+            monkeypatch.setattr(block_ops, "_one_call", lambda *a: False)
+        torch.manual_seed(3)
+        ops.set_dropout_rng_state({"salt": 0, "state": {("cuda", torch.cuda.current_device()): 5}})
+        model.zero_grad_arena()
+        out = model(idx[:, :-1], idx[:, 1:])
+        loss = out[0] if isinstance(out, tuple) else out
+        loss.backward()
+        _status_ok()
+        a = model.arena
+        results.append((loss.item(), [t.clone() for t in [g.G for g in a.groups.values()] + [a.head_grad, a.small_grads]]))
+    assert results[0][0] == results[1][0]
+    for x, y in zip(*(r[1] for r in results)):
+        assert (x - y).norm().item() <= 2e-2 * y.norm().item() + 1e-9
